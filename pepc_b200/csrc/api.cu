@@ -604,7 +604,7 @@ int pepcg_traverse_range_device(void* ctx, int64_t t0, int64_t t1, double* d_ex,
                            d_pot, d_work, c->q.p);
   // the range's own keys give the per-tile walk its tiles, as a rank's local keys would
   return traverse_device(c, t1 - t0, c->x.p + t0, c->y.p + t0, c->z.p + t0, c->key.p + t0, false,
-                         d_ex, d_ey, d_ez, d_pot, d_work, c->q.p + t0);
+                         d_ex, d_ey, d_ez, d_pot, d_work, c->q.p + t0, nullptr, c->n);
 }
 
 int pepcg_restore_device(void* ctx, const double* d_in, double* d_out) {

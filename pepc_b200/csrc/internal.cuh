@@ -319,6 +319,10 @@ int host_tiles(Ctx* c, int64_t nt, const int64_t* d_tkeys, int T, int2* d_tiles,
 // the walk.  Only the per-target and group walks without the periodic far
 // field are split (their per-target results do not depend on the split when
 // the interior bounds are multiples of 32).
+//
+// shape_nt: the target count by which the mixed group walk picks its kernel
+// (0: nt).  Chunks and ranges of one target set pass the whole set's count, so
+// that the split does not change a bucket's sums.
 struct ChunkPlan {
   int nchunks = 1;
   const int64_t* bounds = nullptr;  // nchunks + 1 target offsets
@@ -329,7 +333,7 @@ struct ChunkPlan {
 int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const double* tz,
                     const int64_t* tkeys, bool self, double* ex, double* ey, double* ez,
                     double* pot, double* work, const double* tq = nullptr,
-                    const ChunkPlan* plan = nullptr);
+                    const ChunkPlan* plan = nullptr, int64_t shape_nt = 0);
 
 // walk_mixed.cu: the transposed adjoint walk of the mixed 64-target group walk
 int launch_adjoint_group64(Ctx* c, int64_t nt, const double* tx, const double* ty,

@@ -542,7 +542,8 @@ __global__ void k_mac_thresholds(int64_t M, int mode, const int2* __restrict__ m
 int launch_walk_mixed(Ctx* c, int64_t nt, const double* tx, const double* ty, const double* tz,
                       double* ex, double* ey, double* ez, double* pot, double* work,
                       const int2* tiles, int64_t ntiles, bool per_target, const int32_t* tflag,
-                      const int32_t* pstart, const int32_t* npacks, cudaStream_t s, int slot);
+                      const int32_t* pstart, const int32_t* npacks, cudaStream_t s, int slot,
+                      int64_t shape_nt);
 
 const double* grown_charges_if_same(Ctx* c, int64_t nt, const int64_t* d_tkeys) {
   if (!d_tkeys || nt != c->n) return nullptr;
@@ -573,7 +574,8 @@ int prepare_mac(Ctx* c, const double** macb) {
 
 int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const double* tz,
                     const int64_t* tkeys, bool self, double* ex, double* ey, double* ez,
-                    double* pot, double* work, const double* tq, const ChunkPlan* plan) {
+                    double* pot, double* work, const double* tq, const ChunkPlan* plan,
+                    int64_t shape_nt) {
   if (!c->has_tree) {
     c->err = "traverse called without a grown tree";
     return PEPCG_ERR_NO_TREE;
@@ -754,7 +756,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
         int rc = launch_walk_mixed(c, t1 - t0, A.tx, A.ty, A.tz, A.ex, A.ey, A.ez, A.pot, A.work,
                                    walk == PEPCG_WALK_PER_TILE ? A.tiles : nullptr, ntiles,
                                    walk == PEPCG_WALK_PER_TARGET, packed ? c->tflag.p : nullptr,
-                                   pstart, npacks, sk, slot);
+                                   pstart, npacks, sk, slot, shape_nt > 0 ? shape_nt : nt);
         if (rc) return rc;
       }
       if (!cuda_ok(c, cudaGetLastError(), "walk launch")) return PEPCG_ERR_CUDA;
