@@ -398,8 +398,9 @@ int pepcg_destroy(void* ctx) {
   release(c->adj); release(c->fpo2rpo); release(c->rpo2fpo); release(c->nkey);
   release(c->tiles); release(c->counters); release(c->tgt); release(c->tkeys);
   for (void* p : {(void*)c->d_box, (void*)c->d_status, (void*)c->d_small, (void*)c->d_vbox,
-                  (void*)c->d_part, (void*)c->d_mlattice, (void*)c->d_omega, (void*)c->d_mu,
-                  (void*)c->d_fmm_aux, (void*)c->d_factorial})
+                  (void*)c->d_part, (void*)c->d_mlattice, (void*)c->d_lattab, (void*)c->d_latcoef,
+                  (void*)c->d_latpart, (void*)c->d_ofict, (void*)c->d_site, (void*)c->d_site_q,
+                  (void*)c->d_site_n, (void*)c->d_fmm_aux, (void*)c->d_factorial})
     if (p) cudaFree(p);
   for (int i = 0; i < Ctx::kEvents; ++i)
     if (c->ev[i]) cudaEventDestroy(c->ev[i]);
@@ -410,9 +411,9 @@ int pepcg_destroy(void* ctx) {
     if (c->ready[i]) cudaEventDestroy(c->ready[i]);
     if (c->done[i]) cudaEventDestroy(c->done[i]);
   }
-  for (cudaEvent_t e : {c->fork, c->join})
+  for (cudaEvent_t e : {c->fork, c->join, c->lat_ev})
     if (e) cudaEventDestroy(e);
-  for (cudaStream_t t : {c->h2d, c->d2h, c->walk2})
+  for (cudaStream_t t : {c->h2d, c->d2h, c->walk2, c->lat_stream})
     if (t) {
       cudaStreamSynchronize(t);
       cudaStreamDestroy(t);
@@ -471,11 +472,8 @@ int pepcg_grow_tree_device(void* ctx, int64_t n, const double* d_x, const double
   if (!c || !d_x || !d_y || !d_z || !d_q) return PEPCG_ERR_BAD_ARG;
   cudaSetDevice(c->device);
   int rc = grow_device(c, n, d_x, d_y, d_z, d_q);
-  if (rc) return rc;
-  if (c->far_field) {
-    rc = lattice_timestep(c);
-    if (rc && rc != PEPCG_WARN_NOT_NEUTRAL) return rc;
-  }
+  if (c->far_field) rc = lattice_finish(c, rc);  // also after a failed grow: its step may be running
+  if (rc && rc != PEPCG_WARN_NOT_NEUTRAL) return rc;
   c->grow_times_pending = true;  // read the phase events later, without a sync here
   return rc;
 }
@@ -507,11 +505,8 @@ int pepcg_grow_tree(void* ctx, int64_t n, const double* x, const double* y, cons
       !cuda_ok(c, cudaEventRecord(c->join, c->h2d), "H2D q"))
     return drain_copies(c, false), PEPCG_ERR_CUDA;
   int rc = grow_device(c, n, c->in_x.p, c->in_y.p, c->in_z.p, c->in_q.p, c->join);
-  if (rc) return drain_copies(c, false), rc;
-  if (c->far_field) {
-    rc = lattice_timestep(c);
-    if (rc && rc != PEPCG_WARN_NOT_NEUTRAL) return drain_copies(c, false), rc;
-  }
+  if (c->far_field) rc = lattice_finish(c, rc);
+  if (rc && rc != PEPCG_WARN_NOT_NEUTRAL) return drain_copies(c, false), rc;
   c->grow_times_pending = true;
   // Copy the outputs back on the device-to-host stream while the rest of the
   // grow runs on the context stream: the keys and the permutation (the sorted

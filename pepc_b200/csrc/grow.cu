@@ -1321,6 +1321,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
                                                c->d_small, dupcap, dup_range, c->d_box,
                                                c->prm.curve);
   cudaEventRecord(c->ev[2], s);
+  if (c->far_field && !lattice_timestep(c, n, c->ev[2])) return PEPCG_ERR_CUDA;
   if (!cuda_ok(c, cudaEventSynchronize(c->sum_ev), "grow (keys/sort)")) return PEPCG_ERR_CUDA;
   const Ctx::GrowSummary& gs = *c->h_sum;
   for (int k = 0; k < 9; ++k) c->box[k] = gs.box[k];

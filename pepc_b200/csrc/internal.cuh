@@ -187,6 +187,7 @@ struct Ctx {
     uint32_t status;
     int32_t max_level;
     int32_t lvl[kMaxLevel + 1];
+    uint32_t not_neutral;           // the lattice step found a net charge
   };
   GrowSummary* h_sum = nullptr;  // host address
   GrowSummary* d_sum = nullptr;  // its device address
@@ -200,8 +201,19 @@ struct Ctx {
   double* d_vbox = nullptr;   // the same on the device
   double* d_part = nullptr;   // bbox partials (6 * 296)
   double2* d_mlattice = nullptr;  // 861 complex
-  double2* d_omega = nullptr;     // 231 complex
-  double2* d_mu = nullptr;        // 861 complex
+  // expansions of order 20 (231 orders): the harmonics' recurrence and leading
+  // factors, the force coefficients from mu, block partials of the particle sums,
+  // the fictitious charges' harmonics and their sites over all near boxes
+  double* d_lattab = nullptr;
+  double* d_latcoef = nullptr;
+  double* d_latpart = nullptr;
+  double2* d_ofict = nullptr;
+  double* d_site = nullptr;
+  double* d_site_q = nullptr;
+  int4* d_site_n = nullptr;
+  int nsite = 0;
+  cudaStream_t lat_stream = nullptr;  // the time step's kernels, beside the tree build
+  cudaEvent_t lat_ev = nullptr;
   double* d_fmm_aux = nullptr;    // box dipole (3), quad trace, fict (4 x 4), nfict, ...
   double* d_factorial = nullptr;  // 0..80
 
@@ -347,7 +359,9 @@ int adjoint_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const
 
 // ---- lattice.cu ----
 int lattice_prepare(Ctx* c);
-int lattice_timestep(Ctx* c);
+bool lattice_timestep(Ctx* c, int64_t n, cudaEvent_t ready);  // launches
+// waits for the step: the grow's own status if it failed, else PEPCG_OK or the warning
+int lattice_finish(Ctx* c, int grow_rc);
 // walk_plain.cu: per-twig MAC thresholds for mac_select != 0 (nullptr for Barnes-Hut)
 int prepare_mac(Ctx* c, const double** macb);
 // the grown particles' charges when the targets are exactly the grown

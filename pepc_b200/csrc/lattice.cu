@@ -22,6 +22,7 @@
 // Expansions use the flat layout tblinv(l, m) = l(l+1)/2 + m, m >= 0.
 // Compiled with --fmad=false.
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -36,6 +37,7 @@ constexpr int kLenM = 231;
 constexpr int kLenT = 861;
 constexpr int kLMTable = 50;               // unit-cube table order
 constexpr int kMaxIter = 32;
+constexpr int kMaxSites = 256;             // fictitious charges' sites: at most 6^3 for 125 boxes
 
 __device__ __forceinline__ int tblinv(int l, int m) { return l * (l + 1) / 2 + m; }
 
@@ -213,12 +215,12 @@ __global__ void k_lattice_iter(int lt, int lm, const double2* __restrict__ ML,
   while ((l + 1) * (l + 2) / 2 <= idx) ++l;
   int m = idx - l * (l + 1) / 2;
   double2 t = make_double2(0.0, 0.0);
-  for (int j = 0; j <= lt; ++j) {
+  for (int j = 0; j <= min(lm, lt - l); ++j) {  // Mstar ends at lm, ML at lt
     const double sg = (j & 1) ? -1.0 : 1.0;
     for (int k = -j; k <= j; ++k) {
       const int ll = j + l, mm = k + m;
       double2 a = make_double2(0.0, 0.0);
-      if (ll <= lt && abs(mm) <= ll) {
+      if (abs(mm) <= ll) {
         double2 v = ML[tblinv(ll, abs(mm))];
         const double d = scp[ll];
         v = make_double2(v.x / d, v.y / d);  // UL
@@ -256,201 +258,290 @@ __global__ void k_truncate(const double2* __restrict__ src, double2* __restrict_
   dst[idx] = v;
 }
 
-// box dipole and quadrupole trace (calc_box_dipole, :605-630): block partials
-__global__ void k_box_dipole(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
-                             const double* __restrict__ z, const double* __restrict__ q,
-                             double cx, double cy, double cz, double* __restrict__ part) {
-  double a[4] = {0, 0, 0, 0};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    double r0 = x[i] - cx, r1 = y[i] - cy, r2 = z[i] - cz;
-    a[0] = a[0] + q[i] * r0;
-    a[1] = a[1] + q[i] * r1;
-    a[2] = a[2] + q[i] * r2;
-    a[3] = a[3] + q[i] * ((r0 * r0 + r1 * r1) + r2 * r2);
+// ---- time step and far field: solid harmonics by recurrence ----
+//
+// O_lm(x, y, z) = r^l P_lm(cos theta) e^{-im phi} / (l + m)! is a polynomial,
+//   O_lm = L_lm Q_lm(z, r^2) (x - iy)^m,
+//   Q_mm = 1, Q_{l} = z Q_{l-1} - k_lm r^2 Q_{l-2},  k_lm = ((l-1)^2 - m^2) / ((2l-1)(2l-3)),
+//   L_mm = 1 / (2^m m!),  L_lm = L_{l-1,m} (2l - 1) / ((l - m)(l + m)),
+// so an order needs three operations and neither angles, powers nor divisions
+// (the three-term recurrence of the Legendre polynomials in its monic form, stable
+// upwards for m <= l).  The kernels sum the Q (x - iy)^m alone; L_lm enters once, in
+// k_lattice_step and its output.  Explicit fma(): these sums fix no reference bits.
+// 32,768 ions (ncu): omega 988 -> 23 us, the step after it (four launches) 220 -> 56 us,
+// both now beside the tree build, the force 122 -> 36 us; the earlier kernels took
+// sqrt, atan2 and sincos per particle and a division per order, one thread per
+// coefficient of 1,681 terms, and fresh device memory on each call.
+struct LatTables {
+  double k[kLenM];   // recurrence factors, by tblinv(l, m)
+  double L[kLenM];   // leading factors
+};
+
+LatTables lattice_tables() {
+  LatTables t{};
+  double f = 1.0;
+  for (int m = 0; m <= kLM; ++m) {
+    if (m) f /= 2.0 * m;
+    double L = f;
+    for (int l = m; l <= kLM; ++l) {
+      const int i = l * (l + 1) / 2 + m;
+      if (l > m) L = L * (2.0 * l - 1.0) / ((double)(l - m) * (double)(l + m));
+      t.L[i] = L;
+      t.k[i] = l > m + 1 ? ((l - 1.0) * (l - 1.0) - (double)m * m) / ((2.0 * l - 1.0) * (2.0 * l - 3.0)) : 0.0;
+    }
   }
-  __shared__ double sm[4][8];
-  for (int c = 0; c < 4; ++c) {
-    double v = a[c];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) sm[c][threadIdx.x >> 5] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    double v = 0;
-    for (int w = 0; w < 8; ++w) v += sm[threadIdx.x][w];
-    part[4 * blockIdx.x + threadIdx.x] = v;
-  }
+  return t;
 }
 
-// omega_tilde partials (calc_omega_tilde, :514-596).  Lane m (< 21) of each
-// warp takes the order m of every harmonic of its particles: LegendreP's
-// recurrence (:1196-1242) runs once up through l = 20, giving P_l^m for every
-// l >= m in the same operations as a separate call per l; r^l is carried by
-// multiplication and e^{-i m phi} comes from one sincos.  Each block sums a
-// contiguous chunk of particles (warp partials added in shared memory).
-constexpr int kOmChunk = 1024;
-constexpr int kOmWarps = 8;
-__global__ void __launch_bounds__(256) k_omega_partial(int64_t n, const double* __restrict__ x,
-                                                       const double* __restrict__ y,
-                                                       const double* __restrict__ z,
-                                                       const double* __restrict__ q, double cx,
-                                                       double cy, double cz, const double* fact,
-                                                       double2* __restrict__ part) {
-  __shared__ double2 s_acc[kOmWarps][kLenM];
+// Particle sums S_lm = sum q Q_lm (x - iy)^m over l <= 20 (calc_omega_tilde,
+// :514-596, without L_lm), and sum q r^2 (calc_box_dipole's trace, :605-630; the
+// dipole is in S_1m).  The triangle of orders is folded: lane j < 11 of a half
+// warp takes column m = j and then column 21 - j, 21 steps in all, so a half
+// warp covers one particle and every step's accumulator is a register.
+// One block of partials per SM, summed by k_lattice_step in block order.
+constexpr int kOmBlocks = 148;
+constexpr int kOmWarps = 16;
+constexpr int kOmVals = 2 * kLenM + 1;  // re, im per order, then the trace
+constexpr int kOmCols = 11;
+__global__ void __launch_bounds__(32 * kOmWarps, 1)
+    k_omega_sum(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
+                const double* __restrict__ z, const double* __restrict__ q, double cx, double cy,
+                double cz, const double* __restrict__ ktab, double* __restrict__ part) {
+  __shared__ double s_k[kLM + 1][kOmCols];  // by step and lane
+  extern __shared__ double s_sum[];         // [kOmWarps][kOmVals]
+  for (int i = threadIdx.x; i < (kLM + 1) * kOmCols; i += blockDim.x) {
+    const int s = i / kOmCols, j = i % kOmCols;
+    const bool second = j > 0 && s >= kLM + 1 - j;
+    const int m = second ? kLM + 1 - j : j, l = second ? s : j + s;
+    s_k[s][j] = ktab[tblinv(l, m)];
+  }
+  __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int m = lane;
-  const int64_t base = (int64_t)blockIdx.x * kOmChunk;
-  const int cnt = (int)min((int64_t)kOmChunk, n - base);
-  double2 acc[kLM + 1];
+  const int half = lane >> 4, j = lane & 15;
+  double ar[kLM + 1], ai[kLM + 1], tr = 0.0;
 #pragma unroll
-  for (int l = 0; l <= kLM; ++l) acc[l] = make_double2(0.0, 0.0);
-  if (m <= kLM) {
-    for (int i = w; i < cnt; i += kOmWarps) {
-      double sph[3];
-      cart2sph(x[base + i] - cx, y[base + i] - cy, z[base + i] - cz, sph);
-      const double qi = q[base + i];
-      const double xc = sph[1];
-      double sn, cs;
-      sincos((double)m * sph[2], &sn, &cs);
-      const double sg = (m & 1) ? -1.0 : 1.0;
-      double pmm = 1.0;
-      if (m > 0) {
-        const double somx2 = sqrt((1.0 - xc) * (1.0 + xc));
-        double f = 1.0;
-        for (int k = 1; k <= m; ++k) {
-          pmm = (-pmm * f) * somx2;
-          f = f + 2.0;
+  for (int s = 0; s <= kLM; ++s) ar[s] = ai[s] = 0.0;
+  const int64_t nw = (int64_t)gridDim.x * kOmWarps * 2;
+  if (j < kOmCols) {
+    const int swap = j > 0 ? kLM + 1 - j : kLM + 1;  // first step of the second column
+    for (int64_t i = ((int64_t)blockIdx.x * kOmWarps + w) * 2 + half; i < n; i += nw) {
+      const double dx = x[i] - cx, dy = y[i] - cy, dz = z[i] - cz, qi = q[i];
+      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+      // (x - iy)^j and (x - iy)^(21 - j) from the squares
+      double pr = dx, pi = -dy, er = qi, ei = 0.0, fr = qi, fi = 0.0;
+#pragma unroll
+      for (int b = 0; b < 5; ++b) {
+        if ((j >> b) & 1) {
+          const double t = fma(er, pr, -(ei * pi));
+          ei = fma(er, pi, ei * pr);
+          er = t;
+        }
+        if ((swap >> b) & 1) {
+          const double t = fma(fr, pr, -(fi * pi));
+          fi = fma(fr, pi, fi * pr);
+          fr = t;
+        }
+        if (b < 4) {
+          const double t = fma(pr, pr, -(pi * pi));
+          pi = 2.0 * (pr * pi);
+          pr = t;
         }
       }
-      double pmmp1 = 0.0, rl = 1.0;
+      double q1 = 0.0, q2 = 0.0;
 #pragma unroll
-      for (int l = 0; l <= kLM; ++l) {
-        if (l >= m) {
-          double P;
-          if (l == m) {
-            P = pmm;
-          } else if (l == m + 1) {
-            pmmp1 = (xc * (2.0 * m + 1.0)) * pmm;
-            P = pmmp1;
-          } else {
-            const double pll =
-                ((xc * (2.0 * l - 1.0)) * pmmp1 - ((double)(l + m) - 1.0) * pmm) / (double)(l - m);
-            pmm = pmmp1;
-            pmmp1 = pll;
-            P = pll;
-          }
-          const double pt = (sg * P) / fact[l + m];
-          const double amp = (sph[0] > 0.0 || l > 0) ? rl * pt : pt;
-          acc[l] = cadd(acc[l], make_double2(qi * (amp * cs), qi * (amp * -sn)));
+      for (int s = 0; s <= kLM; ++s) {
+        double v;
+        if (s == 0 || s == swap) {
+          v = 1.0;
+          q1 = 0.0;
+          if (s > 0) { er = fr; ei = fi; }
+        } else {
+          v = fma(-(s_k[s][j] * r2), q2, dz * q1);
         }
-        rl = rl * sph[0];
+        ar[s] = fma(v, er, ar[s]);
+        ai[s] = fma(v, ei, ai[s]);
+        q2 = q1;
+        q1 = v;
       }
+      tr = fma(qi, r2, tr);
     }
   }
+  double* out = s_sum + w * kOmVals;
 #pragma unroll
-  for (int l = 0; l <= kLM; ++l)
-    if (m <= l) s_acc[w][tblinv(l, m)] = acc[l];
+  for (int s = 0; s <= kLM; ++s) {
+    const double a = ar[s] + __shfl_down_sync(0xffffffffu, ar[s], 16);
+    const double b = ai[s] + __shfl_down_sync(0xffffffffu, ai[s], 16);
+    if (lane < kOmCols) {
+      const bool second = j > 0 && s >= kLM + 1 - j;
+      const int m = second ? kLM + 1 - j : j, l = second ? s : j + s;
+      out[2 * tblinv(l, m)] = a;
+      out[2 * tblinv(l, m) + 1] = b;
+    }
+  }
+  tr += __shfl_down_sync(0xffffffffu, tr, 16);
+  if (lane == 0) out[2 * kLenM] = tr;
   __syncthreads();
-  for (int idx = threadIdx.x; idx < kLenM; idx += blockDim.x) {
-    double2 t = s_acc[0][idx];
-    for (int ww = 1; ww < kOmWarps; ++ww) t = cadd(t, s_acc[ww][idx]);
-    part[(int64_t)blockIdx.x * kLenM + idx] = t;
+  for (int i = threadIdx.x; i < kOmVals; i += blockDim.x) {
+    double t = s_sum[i];
+    for (int v = 1; v < kOmWarps; ++v) t += s_sum[v * kOmVals + i];
+    part[(int64_t)blockIdx.x * kOmVals + i] = t;
   }
 }
 
-// sum the partials in block order, add the fictitious charges (:536-559),
-// remove a net monopole (:570-573), then mu_cent = M2L(MLattice, omega)
-__global__ void k_omega_final(int nparts, const double2* __restrict__ part, const double* aux,
-                              double cx, double cy, double cz, const double* fact,
-                              double2* __restrict__ omega, uint32_t* status) {
-  const int idx = threadIdx.x;
-  __shared__ double s_fict[4][4];
+struct LatStepArgs {
+  int nparts;
+  const double* part;      // kOmVals per block
+  const double* ktab;      // L_lm at [kLenM, 2 kLenM)
+  const double2* ofict;    // O_lm(x_f - c) of the (up to four) fictitious charges
+  const double2* ML;
+  int per[3];
+  double len[3];           // |t_lattice_p|
+  double fpos[4][3];       // their positions, in the order of :540-552
+  int corr;
+  int nsite;               // merged fictitious sites (lattice_sites)
+  const int4* site_n;      // how often each fictitious charge falls on the site
+  double* aux;             // dipole (3), trace, nfict, -, -, -, (x, y, z, q) of each
+  double* site_q;          // charge of each site
+  double* coef;            // 8 per order l <= 20, for k_lattice_force
+  unsigned int* not_neutral;  // mapped host word
+};
+
+// One block: the particle sums in block order; the fictitious charges from the
+// box dipole (:540-552); omega with a net monopole removed (:570-573);
+// mu_cent = M2L(MLattice, omega) for l <= 20, the orders L2L to l <= 1 reads; and from
+// mu the coefficients by which k_lattice_force takes phi and E from the Q_am:
+// with o = O_am = p + is and mu(-m) folded onto m > 0, for each (a, m)
+//   phi:  f (p u0 - s v0)                        mu(a, m) = u0 + iv0, f = 1 (m = 0) or 2
+//   E_z: -f (p u1 - s v1)                        mu(a + 1, m)
+//   E_x: -(p (u+ - u-) - s (v+ - v-))            mu(a + 1, m +- 1), no u-, v- for m = 0
+//   E_y: -(p (v+ + v-) + s (u+ + u-))
+// (tbl() zeroes what lies beyond l = 20), each times L_am.
+constexpr int kStepThreads = 1024;
+__global__ void __launch_bounds__(kStepThreads, 1) k_lattice_step(LatStepArgs A) {
+  __shared__ double s_v[kOmVals];
+  __shared__ double2 s_om[kLM + 1][2 * kLM + 1];  // orders -l .. l at m + kLM
+  __shared__ double2 s_ml[kLenT], s_mu[kLenM];
+  __shared__ double s_q[4];
   __shared__ int s_nf;
-  if (idx == 0) {
-    s_nf = (int)aux[4];
-    for (int p = 0; p < s_nf; ++p)
-      for (int k = 0; k < 4; ++k) s_fict[p][k] = aux[8 + 4 * p + k];
+  const int tid = threadIdx.x;
+  for (int i = tid; i < kLenT; i += kStepThreads) s_ml[i] = A.ML[i];
+  for (int i = tid; i < kOmVals; i += kStepThreads) {
+    double t = 0.0;
+#pragma unroll 8
+    for (int b = 0; b < A.nparts; ++b) t += A.part[(int64_t)b * kOmVals + i];
+    s_v[i] = t;
   }
   __syncthreads();
-  if (idx >= kLenM) return;
-  int l = 0;
-  while ((l + 1) * (l + 2) / 2 <= idx) ++l;
-  const int m = idx - l * (l + 1) / 2;
-  double2 acc = make_double2(0.0, 0.0);
-  for (int b = 0; b < nparts; ++b) acc = cadd(acc, part[(int64_t)b * kLenM + idx]);
-  for (int p = 0; p < s_nf; ++p) {
-    double s[3];
-    cart2sph(s_fict[p][0] - cx, s_fict[p][1] - cy, s_fict[p][2] - cz, s);
-    double2 o = omultipole(l, m, s, fact);
-    acc = cadd(acc, make_double2(s_fict[p][3] * o.x, s_fict[p][3] * o.y));
-  }
-  if (idx == 0 && hypot(acc.x, acc.y) > 0.0) {
-    acc = make_double2(0.0, 0.0);
-    atomicOr(status, ST_NOT_NEUTRAL);
-  }
-  omega[idx] = acc;
-}
-
-__global__ void k_mu_cent(const double2* __restrict__ ML, const double2* __restrict__ omega,
-                          double2* __restrict__ mu) {
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= kLenT) return;
-  int l = 0;
-  while ((l + 1) * (l + 2) / 2 <= idx) ++l;
-  int m = idx - l * (l + 1) / 2;
-  double2 t = make_double2(0.0, 0.0);
-  for (int j = 0; j <= kLT; ++j) {
-    const double sg = (j & 1) ? -1.0 : 1.0;
-    for (int k = -j; k <= j; ++k) {
-      double2 a = tbl(ML, j + l, k + m, kLT);
-      t = cadd(t, cmul(make_double2(sg * a.x, sg * a.y), tbl(omega, j, k, kLM)));
+  if (tid == 0) {
+    const double a[3] = {s_v[2 * tblinv(1, 1)], -s_v[2 * tblinv(1, 1) + 1], s_v[2 * tblinv(1, 0)]};
+    for (int k = 0; k < 3; ++k) A.aux[k] = a[k];
+    A.aux[3] = s_v[2 * kLenM];
+    int nf = 0;
+    if (A.corr == 2) {
+      double sum = 0.0;
+      for (int p = 0; p < 3; ++p)
+        if (A.per[p]) s_q[nf++] = -a[p] / A.len[p];
+      for (int p = 0; p < nf; ++p) sum = sum + s_q[p];
+      s_q[nf++] = -sum;
     }
-  }
-  mu[idx] = t;
-}
-
-// fictitious charges from the box dipole (single thread; :540-552)
-__global__ void k_fict(int nbp, const double* __restrict__ part, double* aux, int p0, int p1,
-                       int p2, const double* lat, const double* origin, int corr) {
-  if (threadIdx.x != 0) return;
-  double a[4] = {0, 0, 0, 0};
-  for (int b = 0; b < nbp; ++b)
-    for (int c = 0; c < 4; ++c) a[c] += part[4 * b + c];
-  for (int c = 0; c < 4; ++c) aux[c] = a[c];
-  int nf = 0;
-  if (corr == 2) {
-    int per[3] = {p0, p1, p2};
-    double sum = 0.0;
-    for (int p = 0; p < 3; ++p) {
-      if (!per[p]) continue;
-      const double* L = lat + 3 * p;
-      for (int d = 0; d < 3; ++d) aux[8 + 4 * nf + d] = origin[d] + L[d];
-      aux[8 + 4 * nf + 3] = -a[p] / sqrt((L[0] * L[0] + L[1] * L[1]) + L[2] * L[2]);
-      ++nf;
+    for (int p = 0; p < nf; ++p) {
+      for (int k = 0; k < 3; ++k) A.aux[8 + 4 * p + k] = A.fpos[p][k];
+      A.aux[11 + 4 * p] = s_q[p];
     }
-    for (int p = 0; p < nf; ++p) sum = sum + aux[8 + 4 * p + 3];
-    for (int d = 0; d < 3; ++d) aux[8 + 4 * nf + d] = origin[d];
-    aux[8 + 4 * nf + 3] = -sum;
-    ++nf;
+    for (int p = nf; p < 4; ++p) s_q[p] = 0.0;
+    s_nf = nf;
+    A.aux[4] = nf;
   }
-  aux[4] = nf;
+  __syncthreads();
+  for (int i = tid; i < A.nsite; i += kStepThreads) {
+    const int4 c = A.site_n[i];
+    A.site_q[i] = ((c.x * s_q[0] + c.y * s_q[1]) + c.z * s_q[2]) + c.w * s_q[3];
+  }
+  if (tid < kLenM) {
+    int l = 0;
+    while ((l + 1) * (l + 2) / 2 <= tid) ++l;
+    const int m = tid - l * (l + 1) / 2;
+    const double L = A.ktab[kLenM + tid];
+    double2 o = make_double2(L * s_v[2 * tid], L * s_v[2 * tid + 1]);
+    for (int p = 0; p < s_nf; ++p) {
+      const double2 f = A.ofict[p * kLenM + tid];
+      o = cadd(o, make_double2(s_q[p] * f.x, s_q[p] * f.y));
+    }
+    if (tid == 0) {
+      const bool net = hypot(o.x, o.y) > 0.0;
+      *A.not_neutral = net ? 1u : 0u;
+      if (net) o = make_double2(0.0, 0.0);
+    }
+    const double sg = (m & 1) ? -1.0 : 1.0;
+    s_om[l][kLM - m] = make_double2(sg * o.x, -sg * o.y);
+    s_om[l][kLM + m] = o;
+  }
+  __syncthreads();
+  // four threads per output, each its quarter of the j (:912-937)
+  {
+    const int idx = tid >> 2, part = tid & 3;
+    double2 t = make_double2(0.0, 0.0);
+    if (idx < kLenM) {
+      int l = 0;
+      while ((l + 1) * (l + 2) / 2 <= idx) ++l;
+      const int m = idx - l * (l + 1) / 2;
+      for (int j = part; j <= kLM; j += 4) {
+        const double sg = (j & 1) ? -1.0 : 1.0;
+        for (int k = -j; k <= j; ++k) {
+          const double2 a = tbl(s_ml, j + l, k + m, kLT);
+          t = cadd(t, cmul(make_double2(sg * a.x, sg * a.y), s_om[j][kLM + k]));
+        }
+      }
+    }
+    for (int o = 1; o < 4; o <<= 1) {
+      t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+      t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+    }
+    if (part == 0 && idx < kLenM) s_mu[idx] = t;
+  }
+  __syncthreads();
+  if (tid < kLenM) {
+    int a = 0;
+    while ((a + 1) * (a + 2) / 2 <= tid) ++a;
+    const int m = tid - a * (a + 1) / 2;
+    const double L = A.ktab[kLenM + tid], f = m > 0 ? 2.0 * L : L;
+    const double2 m0 = s_mu[tid], m1 = tbl(s_mu, a + 1, m, kLM);
+    const double2 up = tbl(s_mu, a + 1, m + 1, kLM);
+    const double2 dn = m > 0 ? tbl(s_mu, a + 1, m - 1, kLM) : make_double2(0.0, 0.0);
+    double* o = A.coef + 8 * tid;
+    o[0] = f * m0.x;
+    o[1] = -f * m0.y;
+    o[2] = -f * m1.x;
+    o[3] = f * m1.y;
+    o[4] = -L * (up.x - dn.x);
+    o[5] = L * (up.y - dn.y);
+    o[6] = -L * (up.y + dn.y);
+    o[7] = -L * (up.x + dn.x);
+  }
 }
 
-// fmm_sum_lattice_force per target (:766-826)
+// fmm_sum_lattice_force per target (:766-826): phi and E as sums over the orders of
+// Q_am times k_lattice_step's coefficients, (x - iy)^m applied once per m, then
+// the extrinsic correction.  The fictitious charges of all near boxes are
+// merged by site (coinciding ones add, and interior sites cancel and are left
+// out: 46 terms for 27 boxes instead of 108).
 __global__ void __launch_bounds__(128) k_lattice_force(
     int64_t nt, const double* __restrict__ tx, const double* __restrict__ ty,
-    const double* __restrict__ tz, const double2* __restrict__ mu, const double* __restrict__ aux,
-    const double* __restrict__ vbox, int nbox, double cx, double cy, double cz, double volume,
-    int corr, const double* fact, double* ex, double* ey, double* ez, double* pot, int overwrite) {
-  __shared__ double2 s_mu[kLenM];  // only j <= Lmax_multipole entries are read by L2L
-  __shared__ double s_aux[32];
-  __shared__ double s_vb[3 * 125];
-  __shared__ double s_fact[2 * kLM + 1];
-  for (int i = threadIdx.x; i < kLenM; i += blockDim.x) s_mu[i] = mu[i];
-  for (int i = threadIdx.x; i < 32; i += blockDim.x) s_aux[i] = aux[i];
-  for (int i = threadIdx.x; i < 3 * nbox; i += blockDim.x) s_vb[i] = vbox[i];
-  for (int i = threadIdx.x; i <= 2 * kLM; i += blockDim.x) s_fact[i] = fact[i];
+    const double* __restrict__ tz, const double* __restrict__ coef,
+    const double* __restrict__ ktab, const double* __restrict__ aux, int nsite,
+    const double* __restrict__ site, const double* __restrict__ site_q, double cx, double cy,
+    double cz, double volume, int corr, double* ex, double* ey, double* ez, double* pot,
+    int overwrite) {
+  __shared__ double2 s_c[4 * kLenM];
+  __shared__ double s_k[kLenM];
+  __shared__ double4 s_site[kMaxSites];
+  __shared__ double s_aux[4];
+  for (int i = threadIdx.x; i < 4 * kLenM; i += blockDim.x)
+    s_c[i] = reinterpret_cast<const double2*>(coef)[i];
+  for (int i = threadIdx.x; i < kLenM; i += blockDim.x) s_k[i] = ktab[i];
+  for (int i = threadIdx.x; i < nsite; i += blockDim.x)
+    s_site[i] = make_double4(site[3 * i], site[3 * i + 1], site[3 * i + 2], site_q[i]);
+  if (threadIdx.x < 4) s_aux[threadIdx.x] = aux[threadIdx.x];
   __syncthreads();
   const double pi = acos(-1.0);
   const double prefact = (2.0 * pi) / (3.0 * volume);
@@ -458,61 +549,34 @@ __global__ void __launch_bounds__(128) k_lattice_force(
        t += (int64_t)gridDim.x * blockDim.x) {
     const double px = tx[t], py = ty[t], pz = tz[t];
     const double R0 = px - cx, R1 = py - cy, R2 = pz - cz;
-    double s[3];
-    cart2sph(R0, R1, R2, s);
-    // O_R(a, b) at the target (OMultipole, :695-714) times mu, L2L to l <= 1
-    // (:943-976 with max_l = 1): output (l, m') collects O_R(a, b) mu(a + l,
-    // b + m') over |b| <= a <= 20.  The harmonics are generated order by
-    // order: for each m, one sincos, LegendreP's recurrence through a = 20
-    // and r^a by multiplication, and O_R(a, -m) = (-1)^m conj(O_R(a, m)).
-    double2 ms[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+    const double r2 = fma(R0, R0, fma(R1, R1, R2 * R2));
+    double e0 = 0.0, e1 = 0.0, e2 = 0.0, ph = 0.0;
+    double er = 1.0, ei = 0.0;  // (x - iy)^m
     for (int m = 0; m <= kLM; ++m) {
-      double sn, cs;
-      sincos((double)m * s[2], &sn, &cs);
-      const double sg = (m & 1) ? -1.0 : 1.0;
-      const double xc = s[1];
-      double pmm = 1.0;
-      if (m > 0) {
-        const double somx2 = sqrt((1.0 - xc) * (1.0 + xc));
-        double f = 1.0;
-        for (int k = 1; k <= m; ++k) {
-          pmm = (-pmm * f) * somx2;
-          f = f + 2.0;
-        }
-      }
-      double rl = 1.0;
-      for (int k = 0; k < m; ++k) rl = rl * s[0];
-      double pmmp1 = 0.0;
+      double2 c0 = make_double2(0.0, 0.0), c1 = c0, c2 = c0, c3 = c0;
+      double q1 = 1.0, q2 = 0.0;
+#pragma unroll 3
       for (int a = m; a <= kLM; ++a) {
-        double P;
-        if (a == m) {
-          P = pmm;
-        } else if (a == m + 1) {
-          pmmp1 = (xc * (2.0 * m + 1.0)) * pmm;
-          P = pmmp1;
-        } else {
-          const double pll =
-              ((xc * (2.0 * a - 1.0)) * pmmp1 - ((double)(a + m) - 1.0) * pmm) / (double)(a - m);
-          pmm = pmmp1;
-          pmmp1 = pll;
-          P = pll;
+        const int i = tblinv(a, m);
+        if (a > m) {
+          const double v = fma(-(s_k[i] * r2), q2, R2 * q1);
+          q2 = q1;
+          q1 = v;
         }
-        const double pt = (sg * P) / s_fact[a + m];
-        const double amp = (s[0] > 0.0 || a > 0) ? rl * pt : pt;
-        rl = rl * s[0];
-        const double2 o = make_double2(amp * cs, amp * -sn);
-        ms[0] = cadd(ms[0], cmul(o, tbl(s_mu, a, m, kLM)));
-        ms[1] = cadd(ms[1], cmul(o, tbl(s_mu, a + 1, m, kLM)));
-        ms[2] = cadd(ms[2], cmul(o, tbl(s_mu, a + 1, m + 1, kLM)));
-        if (m > 0) {
-          const double2 on = make_double2(sg * o.x, -sg * o.y);
-          ms[0] = cadd(ms[0], cmul(on, tbl(s_mu, a, -m, kLM)));
-          ms[1] = cadd(ms[1], cmul(on, tbl(s_mu, a + 1, -m, kLM)));
-          ms[2] = cadd(ms[2], cmul(on, tbl(s_mu, a + 1, -m + 1, kLM)));
-        }
+        const double2 a0 = s_c[4 * i], a1 = s_c[4 * i + 1], a2 = s_c[4 * i + 2], a3 = s_c[4 * i + 3];
+        c0.x = fma(q1, a0.x, c0.x); c0.y = fma(q1, a0.y, c0.y);
+        c1.x = fma(q1, a1.x, c1.x); c1.y = fma(q1, a1.y, c1.y);
+        c2.x = fma(q1, a2.x, c2.x); c2.y = fma(q1, a2.y, c2.y);
+        c3.x = fma(q1, a3.x, c3.x); c3.y = fma(q1, a3.y, c3.y);
       }
+      ph = fma(er, c0.x, fma(ei, c0.y, ph));
+      e2 = fma(er, c1.x, fma(ei, c1.y, e2));
+      e0 = fma(er, c2.x, fma(ei, c2.y, e0));
+      e1 = fma(er, c3.x, fma(ei, c3.y, e1));
+      const double tr = fma(er, R0, ei * R1);
+      ei = fma(ei, R0, -(er * R1));
+      er = tr;
     }
-    double e0 = -ms[2].x, e1 = -ms[2].y, e2 = -ms[1].x, ph = ms[0].x;
     if (corr == 1) {
       e0 = e0 + (2.0 * prefact) * s_aux[0];
       e1 = e1 + (2.0 * prefact) * s_aux[1];
@@ -520,20 +584,16 @@ __global__ void __launch_bounds__(128) k_lattice_force(
       double rd = (R0 * s_aux[0] + R1 * s_aux[1]) + R2 * s_aux[2];
       ph = (ph - (2.0 * prefact) * rd) + prefact * s_aux[3];
     } else if (corr == 2) {
-      const int nf = (int)s_aux[4];
-      for (int p = 0; p < nf; ++p) {
-        const double fx = s_aux[8 + 4 * p], fy = s_aux[9 + 4 * p], fz = s_aux[10 + 4 * p];
-        const double fq = s_aux[11 + 4 * p];
-        for (int ib = 0; ib < nbox; ++ib) {
-          const double d0 = (px - s_vb[3 * ib]) - fx, d1 = (py - s_vb[3 * ib + 1]) - fy,
-                       d2 = (pz - s_vb[3 * ib + 2]) - fz;
-          double gx, gy, gz, gp;
-          force_leaf64(fq, d0, d1, d2, (d0 * d0 + d1 * d1) + d2 * d2, gx, gy, gz, gp);
-          e0 = e0 + gx;
-          e1 = e1 + gy;
-          e2 = e2 + gz;
-          ph = ph + gp;
-        }
+#pragma unroll 2
+      for (int k = 0; k < nsite; ++k) {
+        const double4 f = s_site[k];
+        const double d0 = px - f.x, d1 = py - f.y, d2 = pz - f.z;
+        const double ri = rsqrt(fma(d0, d0, fma(d1, d1, d2 * d2)));
+        const double qr = f.w * ri, qr3 = qr * (ri * ri);
+        ph += qr;
+        e0 = fma(qr3, d0, e0);
+        e1 = fma(qr3, d1, e1);
+        e2 = fma(qr3, d2, e2);
       }
     }
     if (overwrite) {
@@ -541,6 +601,22 @@ __global__ void __launch_bounds__(128) k_lattice_force(
     } else {
       ex[t] += e0; ey[t] += e1; ez[t] += e2; pot[t] += ph;
     }
+  }
+}
+
+// O_lm(x_f - c) of the fictitious charges, fixed by the lattice: one thread per order
+__global__ void k_fict_harmonics(int nf, const double* __restrict__ pos, double cx, double cy,
+                                 double cz, const double* __restrict__ fact,
+                                 double2* __restrict__ out) {
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= kLenM) return;
+  int l = 0;
+  while ((l + 1) * (l + 2) / 2 <= idx) ++l;
+  const int m = idx - l * (l + 1) / 2;
+  for (int p = 0; p < nf; ++p) {
+    double s[3];
+    cart2sph(pos[3 * p] - cx, pos[3 * p + 1] - cy, pos[3 * p + 2] - cz, s);
+    out[p * kLenM + idx] = omultipole(l, m, s, fact);
   }
 }
 
@@ -560,6 +636,7 @@ __global__ void __launch_bounds__(128) k_lattice_force(
 // direct terms dL/dq_f (0..3), and for the Redlack form dL/d(dipole) (4..6)
 // and dL/d(trace) (7).
 constexpr int kLatAdjChunk = 1024;
+constexpr int kLatAdjWarps = 8;
 __global__ void __launch_bounds__(256) k_latadj_targets(
     int64_t nt, const double* __restrict__ tx, const double* __restrict__ ty,
     const double* __restrict__ tz, const double* __restrict__ gex, const double* __restrict__ gey,
@@ -567,8 +644,8 @@ __global__ void __launch_bounds__(256) k_latadj_targets(
     double cz, double prefact, int corr, const double* __restrict__ aux,
     const double* __restrict__ vbox, int nbox, const double* __restrict__ fact,
     double2* __restrict__ part, double* __restrict__ xpart) {
-  __shared__ double2 s_acc[kOmWarps][kLenM];
-  __shared__ double s_x[kOmWarps][8];
+  __shared__ double2 s_acc[kLatAdjWarps][kLenM];
+  __shared__ double s_x[kLatAdjWarps][8];
   __shared__ double s_aux[32];
   __shared__ double s_vb[3 * 125];
   __shared__ double s_fact[2 * kLM + 1];
@@ -586,7 +663,7 @@ __global__ void __launch_bounds__(256) k_latadj_targets(
 #pragma unroll
   for (int l = 0; l <= kLM; ++l) acc[l] = make_double2(0.0, 0.0);
   double xa[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = w; i < cnt; i += kOmWarps) {
+  for (int i = w; i < cnt; i += kLatAdjWarps) {
     const int64_t t = base + i;
     const double px = tx[t], py = ty[t], pz = tz[t];
     const double gp = gphi[t], g0 = gex[t], g1 = gey[t], g2 = gez[t];
@@ -684,12 +761,12 @@ __global__ void __launch_bounds__(256) k_latadj_targets(
   __syncthreads();
   for (int idx = threadIdx.x; idx < kLenM; idx += blockDim.x) {
     double2 t = s_acc[0][idx];
-    for (int ww = 1; ww < kOmWarps; ++ww) t = cadd(t, s_acc[ww][idx]);
+    for (int ww = 1; ww < kLatAdjWarps; ++ww) t = cadd(t, s_acc[ww][idx]);
     part[(int64_t)blockIdx.x * kLenM + idx] = t;
   }
   if (threadIdx.x < 8) {
     double v = s_x[0][threadIdx.x];
-    for (int ww = 1; ww < kOmWarps; ++ww) v += s_x[ww][threadIdx.x];
+    for (int ww = 1; ww < kLatAdjWarps; ++ww) v += s_x[ww][threadIdx.x];
     xpart[(int64_t)blockIdx.x * 8 + threadIdx.x] = v;
   }
 }
@@ -910,6 +987,29 @@ bool unit_cube(const pepcg_params& p) {  // system_is_unit_cube, module_mirror_b
 
 }  // namespace
 
+// the centre of the lattice cell (:70-73)
+static void lattice_centre(const pepcg_params& p, double c[3]) {
+  for (int d = 0; d < 3; ++d)
+    c[d] = 0.5 * ((p.t_lattice_1[d] + p.t_lattice_2[d]) + p.t_lattice_3[d]) + p.lattice_origin[d];
+}
+
+// The fictitious charges (:540-552): one at origin + t_lattice_p per periodic
+// direction, the last at the origin.  Returns their number (0 unless corr is 2).
+static int fict_positions(const pepcg_params& p, double pos[4][3], int unit[4][3]) {
+  if (p.fmm_extrinsic_correction != 2) return 0;
+  const double* lv[3] = {p.t_lattice_1, p.t_lattice_2, p.t_lattice_3};
+  int nf = 0;
+  for (int k = 0; k <= 3; ++k) {
+    if (k < 3 && !p.periodicity[k]) continue;
+    for (int d = 0; d < 3; ++d) {
+      pos[nf][d] = k < 3 ? p.lattice_origin[d] + lv[k][d] : p.lattice_origin[d];
+      unit[nf][d] = k == d;
+    }
+    ++nf;
+  }
+  return nf;
+}
+
 int lattice_prepare(Ctx* c) {
   const pepcg_params& p = c->prm;
   cudaStream_t s = c->stream;
@@ -921,25 +1021,90 @@ int lattice_prepare(Ctx* c) {
   std::vector<double> hf(2 * lt + 2), hs(lt + 1);
   for (int i = 0; i < (int)hf.size(); ++i) hf[i] = host_factorial(i);
   for (int l = 0; l <= lt; ++l) hs[l] = std::pow((double)(2 * ws + 1), (double)(l + 1));
+  // the sites of the fictitious charges over all near boxes, by lattice index: a
+  // site that every charge reaches equally often carries their sum, zero
+  double fpos[4][3];
+  int unit[4][3];
+  const int nf = fict_positions(p, fpos, unit);
+  struct Site {
+    int at[3];
+    double pos[3];
+    int n[4];
+  };
+  std::vector<Site> sites;
+  int sw[3];
+  for (int d = 0; d < 3; ++d) sw[d] = p.periodicity[d] ? ws : 0;
+  const double* lv[3] = {p.t_lattice_1, p.t_lattice_2, p.t_lattice_3};
+  for (int f = 0; f < nf; ++f)
+    for (int i = -sw[0]; i <= sw[0]; ++i)
+      for (int j = -sw[1]; j <= sw[1]; ++j)
+        for (int k = -sw[2]; k <= sw[2]; ++k) {
+          const int at[3] = {i + unit[f][0], j + unit[f][1], k + unit[f][2]};
+          Site* hit = nullptr;
+          for (Site& q : sites)
+            if (q.at[0] == at[0] && q.at[1] == at[1] && q.at[2] == at[2]) hit = &q;
+          if (!hit) {
+            Site q{{at[0], at[1], at[2]}, {0, 0, 0}, {0, 0, 0, 0}};
+            for (int d = 0; d < 3; ++d)
+              q.pos[d] = (((double)i * lv[0][d] + (double)j * lv[1][d]) + (double)k * lv[2][d]) + fpos[f][d];
+            sites.push_back(q);
+            hit = &sites.back();
+          }
+          ++hit->n[f];
+        }
+  std::vector<double> hpos;
+  std::vector<int4> hn;
+  for (const Site& q : sites) {
+    bool cancels = true;
+    for (int f = 1; f < nf; ++f) cancels = cancels && q.n[f] == q.n[0];
+    if (cancels) continue;
+    hpos.insert(hpos.end(), q.pos, q.pos + 3);
+    hn.push_back(make_int4(q.n[0], q.n[1], q.n[2], q.n[3]));
+  }
+  c->nsite = (int)hn.size();
+  if (c->nsite > kMaxSites) {
+    c->err = "lattice: too many fictitious charge sites";
+    return PEPCG_ERR_UNSUPPORTED;
+  }
+  const LatTables tab = lattice_tables();
   double2 *mstar = nullptr, *lstar = nullptr, *ml0 = nullptr, *ml1 = nullptr;
-  double *scratch = nullptr, *d_scp = nullptr;
+  double *scratch = nullptr, *d_scp = nullptr, *d_fpos = nullptr;
   const int64_t cnt = (int64_t)nb * (nb - 1);
   const size_t scratch_n = (size_t)lent * 2 * (cnt > nb ? cnt : nb);
   bool ok = cuda_ok(c, cudaMalloc((void**)&c->d_factorial, hf.size() * 8), "fmm") &&
             cuda_ok(c, cudaMalloc((void**)&c->d_mlattice, kLenT * 16), "fmm") &&
-            cuda_ok(c, cudaMalloc((void**)&c->d_omega, kLenM * 16), "fmm") &&
-            cuda_ok(c, cudaMalloc((void**)&c->d_mu, kLenT * 16), "fmm") &&
+            cuda_ok(c, cudaMalloc((void**)&c->d_lattab, sizeof(LatTables)), "fmm") &&
+            cuda_ok(c, cudaMalloc((void**)&c->d_latcoef, 8 * kLenM * 8), "fmm") &&
+            cuda_ok(c, cudaMalloc((void**)&c->d_latpart, (size_t)kOmBlocks * kOmVals * 8), "fmm") &&
+            cuda_ok(c, cudaMalloc((void**)&c->d_ofict, 4 * kLenM * 16), "fmm") &&
+            cuda_ok(c, cudaMalloc((void**)&c->d_site, 3 * kMaxSites * 8), "fmm") &&
+            cuda_ok(c, cudaMalloc((void**)&c->d_site_q, kMaxSites * 8), "fmm") &&
+            cuda_ok(c, cudaMalloc((void**)&c->d_site_n, kMaxSites * sizeof(int4)), "fmm") &&
             cuda_ok(c, cudaMalloc((void**)&c->d_fmm_aux, 64 * 8), "fmm") &&
+            cuda_ok(c, cudaStreamCreateWithFlags(&c->lat_stream, cudaStreamNonBlocking), "fmm") &&
+            cuda_ok(c, cudaEventCreateWithFlags(&c->lat_ev, cudaEventDisableTiming), "fmm") &&
+            cuda_ok(c, cudaFuncSetAttribute(k_omega_sum, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            kOmWarps * kOmVals * 8), "fmm") &&
             cuda_ok(c, cudaMalloc((void**)&mstar, lenm * 16), "fmm") &&
             cuda_ok(c, cudaMalloc((void**)&lstar, lent * 16), "fmm") &&
             cuda_ok(c, cudaMalloc((void**)&ml0, lent * 16), "fmm") &&
             cuda_ok(c, cudaMalloc((void**)&ml1, lent * 16), "fmm") &&
             cuda_ok(c, cudaMalloc((void**)&d_scp, (lt + 1) * 8), "fmm") &&
+            cuda_ok(c, cudaMalloc((void**)&d_fpos, 4 * 3 * 8), "fmm") &&
             cuda_ok(c, cudaMalloc((void**)&scratch, scratch_n * 8), "fmm scratch");
   if (ok) {
+    double ctr[3];
+    lattice_centre(p, ctr);
     cudaMemcpyAsync(c->d_factorial, hf.data(), hf.size() * 8, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(d_scp, hs.data(), hs.size() * 8, cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(c->d_lattab, &tab, sizeof(tab), cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(d_fpos, fpos, nf * 3 * 8, cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(c->d_site, hpos.data(), hpos.size() * 8, cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(c->d_site_n, hn.data(), hn.size() * sizeof(int4), cudaMemcpyHostToDevice, s);
     cudaMemsetAsync(c->d_fmm_aux, 0, 64 * 8, s);
+    COUNT_LAUNCH();
+    k_fict_harmonics<<<(kLenM + 63) / 64, 64, 0, s>>>(nf, d_fpos, ctr[0], ctr[1], ctr[2],
+                                                     c->d_factorial, c->d_ofict);
     COUNT_LAUNCH();
     k_mstar<<<(lenm + 63) / 64, 64, 0, s>>>(lm, nb, c->d_vbox, c->d_factorial, scratch, mstar);
     COUNT_LAUNCH();
@@ -955,78 +1120,77 @@ int lattice_prepare(Ctx* c) {
     ok = cuda_ok(c, cudaGetLastError(), "lattice coefficients") &&
          cuda_ok(c, cudaStreamSynchronize(s), "lattice coefficients");
   }
-  for (void* q : {(void*)mstar, (void*)lstar, (void*)ml0, (void*)ml1, (void*)scratch, (void*)d_scp})
+  for (void* q : {(void*)mstar, (void*)lstar, (void*)ml0, (void*)ml1, (void*)scratch, (void*)d_scp,
+                  (void*)d_fpos})
     if (q) cudaFree(q);
   return ok ? PEPCG_OK : PEPCG_ERR_CUDA;
 }
 
-int lattice_timestep(Ctx* c) {
+// fmm_framework_timestep on a stream of its own, beside the tree build: the n
+// particles stand in key order once event `ready` has passed.  lattice_finish
+// waits for it before the grow returns, so what follows needs no ordering.
+bool lattice_timestep(Ctx* c, int64_t n, cudaEvent_t ready) {
   const pepcg_params& p = c->prm;
-  cudaStream_t s = c->stream;
-  const double cx = 0.5 * ((p.t_lattice_1[0] + p.t_lattice_2[0]) + p.t_lattice_3[0]) + p.lattice_origin[0];
-  const double cy = 0.5 * ((p.t_lattice_1[1] + p.t_lattice_2[1]) + p.t_lattice_3[1]) + p.lattice_origin[1];
-  const double cz = 0.5 * ((p.t_lattice_1[2] + p.t_lattice_2[2]) + p.t_lattice_3[2]) + p.lattice_origin[2];
-  const int64_t n = c->n;
-  const int nbp = 148;
-  const int64_t nom = (n + kOmChunk - 1) / kOmChunk;
-  double* part = nullptr;
-  double2* opart = nullptr;
-  double* d_lat = nullptr;
-  bool ok = cuda_ok(c, cudaMallocAsync((void**)&part, 4 * nbp * 8, s), "fmm") &&
-            cuda_ok(c, cudaMallocAsync((void**)&opart, nom * kLenM * 16, s), "fmm") &&
-            cuda_ok(c, cudaMallocAsync((void**)&d_lat, 12 * 8, s), "fmm");
-  if (!ok) return PEPCG_ERR_OOM;
-  double lat[12];
+  cudaStream_t s = c->lat_stream;
+  if (!cuda_ok(c, cudaStreamWaitEvent(s, ready, 0), "lattice timestep")) return false;
+  double ctr[3];
+  lattice_centre(p, ctr);
+  const int blocks = (int)std::min<int64_t>(kOmBlocks, (n + 2 * kOmWarps - 1) / (2 * kOmWarps));
+  COUNT_LAUNCH();
+  k_omega_sum<<<blocks, 32 * kOmWarps, kOmWarps * kOmVals * 8, s>>>(
+      n, c->x.p, c->y.p, c->z.p, c->q.p, ctr[0], ctr[1], ctr[2], c->d_lattab, c->d_latpart);
+  LatStepArgs A{};
+  A.nparts = blocks;
+  A.part = c->d_latpart;
+  A.ktab = c->d_lattab;
+  A.ofict = c->d_ofict;
+  A.ML = c->d_mlattice;
+  const double* lv[3] = {p.t_lattice_1, p.t_lattice_2, p.t_lattice_3};
   for (int d = 0; d < 3; ++d) {
-    lat[d] = p.t_lattice_1[d];
-    lat[3 + d] = p.t_lattice_2[d];
-    lat[6 + d] = p.t_lattice_3[d];
-    lat[9 + d] = p.lattice_origin[d];
+    A.per[d] = p.periodicity[d];
+    A.len[d] = std::sqrt((lv[d][0] * lv[d][0] + lv[d][1] * lv[d][1]) + lv[d][2] * lv[d][2]);
   }
-  cudaMemcpyAsync(d_lat, lat, 12 * 8, cudaMemcpyHostToDevice, s);
-  cudaMemsetAsync(c->d_status, 0, 4, s);
+  int unit[4][3];
+  fict_positions(p, A.fpos, unit);
+  A.corr = p.fmm_extrinsic_correction;
+  A.nsite = c->nsite;
+  A.site_n = c->d_site_n;
+  A.aux = c->d_fmm_aux;
+  A.site_q = c->d_site_q;
+  A.coef = c->d_latcoef;
+  A.not_neutral = &c->d_sum->not_neutral;
   COUNT_LAUNCH();
-  k_box_dipole<<<nbp, 256, 0, s>>>(n, c->x.p, c->y.p, c->z.p, c->q.p, cx, cy, cz, part);
-  COUNT_LAUNCH();
-  k_fict<<<1, 32, 0, s>>>(nbp, part, c->d_fmm_aux, p.periodicity[0], p.periodicity[1],
-                         p.periodicity[2], d_lat, d_lat + 9, p.fmm_extrinsic_correction);
-  COUNT_LAUNCH();
-  k_omega_partial<<<(unsigned)nom, 256, 0, s>>>(n, c->x.p, c->y.p, c->z.p, c->q.p, cx, cy, cz,
-                                                c->d_factorial, opart);
-  COUNT_LAUNCH();
-  k_omega_final<<<1, 256, 0, s>>>((int)nom, opart, c->d_fmm_aux, cx, cy, cz, c->d_factorial,
-                                  c->d_omega, c->d_status);
-  COUNT_LAUNCH();
-  k_mu_cent<<<(kLenT + 127) / 128, 128, 0, s>>>(c->d_mlattice, c->d_omega, c->d_mu);
-  uint32_t st = 0;
-  ok = cuda_ok(c, cudaGetLastError(), "lattice timestep") &&
-       cuda_ok(c, cudaMemcpyAsync(&st, c->d_status, 4, cudaMemcpyDeviceToHost, s), "status");
-  cudaFreeAsync(part, s);
-  cudaFreeAsync(opart, s);
-  cudaFreeAsync(d_lat, s);
-  ok = ok && cuda_ok(c, cudaStreamSynchronize(s), "lattice timestep");
-  if (!ok) return PEPCG_ERR_CUDA;
-  return st ? status_to_code(c, st) : PEPCG_OK;
+  k_lattice_step<<<1, kStepThreads, 0, s>>>(A);
+  return cuda_ok(c, cudaGetLastError(), "lattice timestep") &&
+         cuda_ok(c, cudaEventRecord(c->lat_ev, s), "lattice timestep");
+}
+
+int lattice_finish(Ctx* c, int grow_rc) {
+  if (grow_rc) {
+    cudaEventSynchronize(c->lat_ev);
+    return grow_rc;
+  }
+  if (!cuda_ok(c, cudaEventSynchronize(c->lat_ev), "lattice timestep")) return PEPCG_ERR_CUDA;
+  return c->h_sum->not_neutral ? status_to_code(c, ST_NOT_NEUTRAL) : PEPCG_OK;
 }
 
 int lattice_add(Ctx* c, int64_t nt, const double* tx, const double* ty, const double* tz,
                 double* ex, double* ey, double* ez, double* pot, bool overwrite) {
   const pepcg_params& p = c->prm;
   cudaStream_t s = c->stream;
-  const double cx = 0.5 * ((p.t_lattice_1[0] + p.t_lattice_2[0]) + p.t_lattice_3[0]) + p.lattice_origin[0];
-  const double cy = 0.5 * ((p.t_lattice_1[1] + p.t_lattice_2[1]) + p.t_lattice_3[1]) + p.lattice_origin[1];
-  const double cz = 0.5 * ((p.t_lattice_1[2] + p.t_lattice_2[2]) + p.t_lattice_3[2]) + p.lattice_origin[2];
+  double ctr[3];
+  lattice_centre(p, ctr);
   const double* a = p.t_lattice_1;
   const double* b = p.t_lattice_2;
   const double* cc = p.t_lattice_3;
   double cr[3] = {a[1] * b[2] - a[2] * b[1], a[2] * b[0] - a[0] * b[2], a[0] * b[1] - a[1] * b[0]};
   const double volume = std::fabs((cr[0] * cc[0] + cr[1] * cc[1]) + cr[2] * cc[2]);
-  unsigned blocks = (unsigned)((nt + 127) / 128);
-  if (blocks > 148 * 16) blocks = 148 * 16;
+  unsigned blocks = (unsigned)std::min<int64_t>((nt + 127) / 128, 148 * 6);
   COUNT_LAUNCH();
-  k_lattice_force<<<blocks, 128, 0, s>>>(nt, tx, ty, tz, c->d_mu, c->d_fmm_aux, c->d_vbox, c->nboxes,
-                                         cx, cy, cz, volume, p.fmm_extrinsic_correction,
-                                         c->d_factorial, ex, ey, ez, pot, overwrite ? 1 : 0);
+  k_lattice_force<<<blocks, 128, 0, s>>>(nt, tx, ty, tz, c->d_latcoef, c->d_lattab, c->d_fmm_aux,
+                                         c->nsite, c->d_site, c->d_site_q, ctr[0], ctr[1], ctr[2],
+                                         volume, p.fmm_extrinsic_correction, ex, ey, ez, pot,
+                                         overwrite ? 1 : 0);
   return cuda_ok(c, cudaGetLastError(), "lattice force") ? PEPCG_OK : PEPCG_ERR_CUDA;
 }
 
