@@ -345,7 +345,7 @@ int pepcg_create(void** out, const pepcg_params* p) {
   for (int i = 0; i < Ctx::kEvents; ++i) cudaEventCreate(&c->ev[i]);
   bool ok = cuda_ok(nullptr, cudaMalloc((void**)&c->d_box, 64 * sizeof(double)), "box") &&
             cuda_ok(nullptr, cudaMalloc((void**)&c->d_status, 16), "status") &&
-            cuda_ok(nullptr, cudaMalloc((void**)&c->d_small, 16 * sizeof(unsigned long long)), "small") &&
+            cuda_ok(nullptr, cudaMalloc((void**)&c->d_small, 32 * sizeof(unsigned long long)), "small") &&
             cuda_ok(nullptr, cudaMalloc((void**)&c->d_vbox, 3 * 125 * sizeof(double)), "vbox") &&
             cuda_ok(nullptr, cudaMalloc((void**)&c->d_part, 6 * 512 * sizeof(double)), "part") &&
             cuda_ok(nullptr, cudaHostAlloc((void**)&c->h_sum, sizeof(Ctx::GrowSummary),

@@ -525,6 +525,193 @@ void sort_pass(int64_t n, const uint64_t* kin, const int32_t* vin, uint64_t* kou
 }
 
 // ---------------------------------------------------------------------------
+// All LSD passes in one cooperative launch, for arrays of few tiles.
+//
+// Up to 148 tiles the 28 launches of the passes above are short of work: at
+// 16,411 keys the sort phase took 172 us with them and takes 68 us with this, most of
+// the difference the start and end of kernels that run for 1-2 us.  Here every tile has a resident block that keeps it through all
+// passes, with two grid barriers per pass: one once the tiles' digit counts are
+// written, after which each block sums the count columns itself (thread d digit d,
+// coalesced over the tiles), one once the pass's output is written.  A pass reads
+// its keys and indices once (registers): the ranking's per-warp counts are also
+// the tile's histogram.  The sort order and stability are the passes' above.
+// Tiles are 512 kPer keys: small tiles spread a small array over more SMs and
+// shorten each warp's chain of ranking rounds; the column sums grow with the
+// tiles, so larger arrays take larger ones.
+// For grow keys the sorted keys and the equal neighbours (k_sorted_keys' output)
+// follow in the same launch.
+// ---------------------------------------------------------------------------
+constexpr int kCoopTiles = 148;
+struct CoopSortArgs {
+  int64_t n;
+  uint64_t *k0, *k1;  // input in k0, v0; the passes alternate
+  int32_t *v0, *v1;
+  uint32_t* hist;  // kMaxDigits per tile
+  unsigned* word;  // grid barrier
+  uint32_t* status;
+  int64_t* ko;     // grow keys: the sorted keys, twice
+  int64_t* korig;
+  unsigned long long* dupcount;
+  int32_t* duplist;
+  int dupcap;
+};
+
+template <int kPer>
+constexpr int coop_smem() {
+  return 512 * kPer * 12 + 2 * kMaxDigits * 4 + kWarpsSort * kMaxDigits * 2;
+}
+
+// exclusive scan of v over the block's first D threads (whole warps); wtot: one slot per warp
+template <int D>
+__device__ __forceinline__ uint32_t digit_scan(uint32_t v, uint32_t* wtot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) wtot[warp] = x;
+  __syncthreads();
+  const uint32_t t = lane < D / 32 && lane < warp ? wtot[lane] : 0u;
+  const uint32_t pre = __reduce_add_sync(0xffffffffu, t);
+  __syncthreads();
+  return pre + x - v;
+}
+
+template <int kBits, int kPer>
+__device__ __forceinline__ bool coop_pass(const CoopSortArgs& A, int from, int shift, int cnt,
+                                          uint64_t* sk, int32_t* sv, uint32_t* lstart,
+                                          uint32_t* gbase, uint16_t (*wcnt)[kMaxDigits],
+                                          uint32_t* wtot, unsigned& barriers) {
+  constexpr int D = 1 << kBits;
+  constexpr int kTile = 512 * kPer, kWarpKeys = 32 * kPer;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const int nb = gridDim.x;
+  const int64_t base = (int64_t)blockIdx.x * kTile;
+  const uint64_t* kin = (from ? A.k1 : A.k0) + base;
+  const int32_t* vin = (from ? A.v1 : A.v0) + base;
+  uint64_t kr[kPer];
+  int32_t vr[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int i = warp * kWarpKeys + j * 32 + lane;
+    kr[j] = i < cnt ? __ldcg(reinterpret_cast<const unsigned long long*>(kin) + i) : 0ull;
+    vr[j] = i < cnt ? __ldcg(vin + i) : 0;
+  }
+  for (int i = tid; i < kWarpsSort * D; i += kScatterThreads) wcnt[i / D][i % D] = 0;
+  __syncthreads();
+  int rk[kPer];
+  uint16_t* my = wcnt[warp];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const bool valid = warp * kWarpKeys + j * 32 + lane < cnt;
+    const int d = (int)((kr[j] >> shift) & (D - 1));
+    unsigned peers = __ballot_sync(0xffffffffu, valid);
+    if (!valid) peers = ~peers;
+#pragma unroll
+    for (int bit = 0; bit < kBits; ++bit) {
+      const bool on = (d >> bit) & 1;
+      const unsigned m = __ballot_sync(0xffffffffu, on);
+      peers &= on ? m : ~m;
+    }
+    const int leader = __ffs(peers) - 1;
+    uint32_t c0 = 0;
+    if (valid && lane == leader) c0 = my[d];
+    c0 = __shfl_sync(0xffffffffu, c0, leader);
+    rk[j] = (int)c0 + __popc(peers & lt);
+    if (valid && lane == leader) my[d] = (uint16_t)(c0 + __popc(peers));
+    __syncwarp();
+  }
+  __syncthreads();
+  uint32_t run = 0;
+  if (tid < D) {
+#pragma unroll
+    for (int w = 0; w < kWarpsSort; ++w) {
+      const uint32_t t = wcnt[w][tid];
+      wcnt[w][tid] = (uint16_t)run;
+      run += t;
+    }
+    __stcg(A.hist + (int64_t)blockIdx.x * kMaxDigits + tid, run);
+  }
+  const uint32_t ls = digit_scan<D>(run, wtot);
+  if (tid < D) lstart[tid] = ls;
+  if (nb > 1 && !grid_barrier(A.word, ++barriers * nb, A.status)) return false;
+  uint32_t tot = 0, pre = 0;
+  if (tid < D) {
+    const uint32_t* col = A.hist + tid;
+#pragma unroll 8
+    for (int b = 0; b < nb; ++b) {
+      const uint32_t v = __ldcg(col + (int64_t)b * kMaxDigits);
+      if (b < (int)blockIdx.x) pre += v;
+      tot += v;
+    }
+  }
+  const uint32_t gs = digit_scan<D>(tot, wtot);
+  if (tid < D) gbase[tid] = gs + pre;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (warp * kWarpKeys + j * 32 + lane < cnt) {
+      const int d = (int)((kr[j] >> shift) & (D - 1));
+      const int pos = (int)(lstart[d] + wcnt[warp][d]) + rk[j];
+      sk[pos] = kr[j];
+      sv[pos] = vr[j];
+    }
+  }
+  __syncthreads();
+  uint64_t* kout = from ? A.k0 : A.k1;
+  int32_t* vout = from ? A.v0 : A.v1;
+  for (int i = tid; i < cnt; i += kScatterThreads) {
+    const uint64_t k = sk[i];
+    const int d = (int)((k >> shift) & (D - 1));
+    const uint32_t dst = gbase[d] + (uint32_t)(i - (int)lstart[d]);
+    kout[dst] = k;
+    vout[dst] = sv[i];
+  }
+  // the output is complete; also, sk, sv and the counts may be written again
+  if (nb > 1) return grid_barrier(A.word, ++barriers * nb, A.status);
+  __syncthreads();
+  return true;
+}
+
+template <bool kGrow, int kPer>
+__global__ void __launch_bounds__(kScatterThreads, 1) k_sort_coop(CoopSortArgs A) {
+  constexpr int kTile = 512 * kPer;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ uint32_t wtot[32];
+  uint64_t* sk = reinterpret_cast<uint64_t*>(smem);
+  int32_t* sv = reinterpret_cast<int32_t*>(sk + kTile);
+  uint32_t* lstart = reinterpret_cast<uint32_t*>(sv + kTile);
+  uint32_t* gbase = lstart + kMaxDigits;
+  uint16_t(*wcnt)[kMaxDigits] = reinterpret_cast<uint16_t(*)[kMaxDigits]>(gbase + kMaxDigits);
+  const int64_t base = (int64_t)blockIdx.x * kTile;
+  const int cnt = (int)min((int64_t)kTile, A.n - base);
+  unsigned barriers = 0;
+  int from = 0;
+  if (kGrow) {  // bits 0 .. 59 in four passes of 9 bits and three of 8
+    for (int shift = 0; shift < 36; shift += 9, from ^= 1)
+      if (!coop_pass<9, kPer>(A, from, shift, cnt, sk, sv, lstart, gbase, wcnt, wtot, barriers)) return;
+    for (int shift = 36; shift < 60; shift += 8, from ^= 1)
+      if (!coop_pass<8, kPer>(A, from, shift, cnt, sk, sv, lstart, gbase, wcnt, wtot, barriers)) return;
+    const unsigned long long* ks = reinterpret_cast<const unsigned long long*>(from ? A.k1 : A.k0);
+    for (int j = threadIdx.x; j < cnt; j += kScatterThreads) {
+      const int64_t i = base + j;
+      const uint64_t k = __ldcg(ks + i);
+      A.ko[i] = (int64_t)k;
+      A.korig[i] = (int64_t)k;
+      if (i + 1 < A.n && __ldcg(ks + i + 1) == k) {
+        const unsigned long long slot = atomicAdd(A.dupcount, 1ull);
+        if (slot < (unsigned long long)A.dupcap) A.duplist[slot] = (int32_t)i;
+      }
+    }
+  } else {
+    for (int shift = 0; shift < 64; shift += 8, from ^= 1)
+      if (!coop_pass<8, kPer>(A, from, shift, cnt, sk, sv, lstart, gbase, wcnt, wtot, barriers)) return;
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Permute the payload into key order, flag duplicates (module_domains.f90:199-234)
 // ---------------------------------------------------------------------------
 // The sorted keys (also kept as the keys before the duplicate fix), and the
@@ -1173,6 +1360,53 @@ void exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, int32_t* tmp
   exclusive_scan<int32_t>(in, out, n, tmp, s);
 }
 
+// k_sort_coop for arrays of up to 148 tiles; false: not launched (see lsd_sort).
+// The barrier word must be zero.
+template <bool kGrow>
+static bool coop_sort(Ctx* c, int64_t n, int dupcap, cudaStream_t s) {
+  CoopSortArgs A{};
+  A.n = n;
+  A.k0 = c->skey.p; A.k1 = c->skey_alt.p;
+  A.v0 = c->sval.p; A.v1 = c->sval_alt.p;
+  A.hist = c->hist.p;
+  A.word = c->barrier_word(0);
+  A.status = c->d_status;
+  A.ko = c->key.p;
+  A.korig = c->orig_key.p;
+  A.dupcount = c->d_small;
+  A.duplist = c->dup_list.p;
+  A.dupcap = dupcap;
+  auto go = [&](auto kern, int per, int smem) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      return false;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)((n + 512 * per - 1) / (512 * per)));
+    cfg.blockDim = dim3(kScatterThreads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, A) != cudaSuccess) {
+      cudaGetLastError();  // the passes one by one instead
+      return false;
+    }
+    COUNT_LAUNCH();
+    return true;
+  };
+  const int64_t rows = (n + 511) / 512;
+  // sort phase, us, tiles of 1,024 / 2,048 / 4,096 keys: 4,099 keys 57 / 65 / 78,
+  // 16,411: 68 / 69 / 88, 60,013: 90 / 90 / 102, 100,003: 107 / 94 / 100, 200,003: - / 123
+  // / 116, 600,000: - / - / 166 (the passes one by one: 164, 172, 172, 172, 177, 184)
+  const int per = rows <= 64 ? 2 : rows <= 256 ? 4 : 8;
+  if ((rows + per - 1) / per > kCoopTiles) return false;
+  if (per == 2) return go(k_sort_coop<kGrow, 2>, 2, coop_smem<2>());
+  if (per == 4) return go(k_sort_coop<kGrow, 4>, 4, coop_smem<4>());
+  return go(k_sort_coop<kGrow, 8>, 8, coop_smem<8>());
+}
+
 // The LSD radix sort of the n (key, index) pairs in skey / sval, ping-ponging
 // through skey_alt / sval_alt.  Grow keys (placeholder bit 60, key bits 0..59)
 // take 7 passes over bits 0..59, any other 64-bit keys 8 passes of 8 bits; the
@@ -1246,7 +1480,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
       !ensure(c, c->q, n, "q") || !ensure(c, c->key, n, "key") || !ensure(c, c->perm, n, "perm") ||
       !ensure(c, c->skey, n, "skey") || !ensure(c, c->skey_alt, n, "skey_alt") ||
       !ensure(c, c->sval, n, "sval") || !ensure(c, c->sval_alt, n, "sval_alt") ||
-      !ensure(c, c->hist, kMaxDigits * nblk_sort + 1, "hist") ||
+      !ensure(c, c->hist, std::max<int64_t>(kMaxDigits * nblk_sort, kMaxDigits * kCoopTiles) + 1, "hist") ||
       !ensure(c, c->scan_tmp, 2 * ((kMaxDigits * nblk_sort + n) / 2048 + 64), "scan_tmp") ||
       !ensure(c, c->orig_key, n, "orig_key") || !ensure(c, c->dup_list, dupcap, "dup_list") ||
       !ensure(c, c->lev, n, "lev") || !ensure(c, c->lcpn, n, "lcpn") ||
@@ -1257,7 +1491,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
     return PEPCG_ERR_OOM;
 
   if (!cuda_ok(c, cudaMemsetAsync(c->d_status, 0, sizeof(uint32_t), s), "memset status") ||
-      !cuda_ok(c, cudaMemsetAsync(c->d_small, 0, 8 * sizeof(unsigned long long), s), "memset") ||
+      !cuda_ok(c, cudaMemsetAsync(c->d_small, 0, 32 * sizeof(unsigned long long), s), "memset") ||
       !cuda_ok(c, cudaMemsetAsync(c->lvlcnt.p, 0, 64 * sizeof(int32_t), s), "memset lvl"))
     return PEPCG_ERR_CUDA;
 
@@ -1277,13 +1511,17 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
                                                               c->skey.p, c->sval.p, c->packed.p);
   cudaEventRecord(c->ev[1], s);
   // sort: 7 LSD passes over the 60 key bits below the placeholder; the result
-  // is in skey / sval
-  lsd_sort(c, n, true, s);
-  uint64_t* kin = c->skey.p;
+  // is in skey / sval, the sorted keys in key / orig_key
+  if (coop_sort<true>(c, n, dupcap, s)) {
+    std::swap(c->skey, c->skey_alt);  // an odd number of passes
+    std::swap(c->sval, c->sval_alt);
+  } else {
+    lsd_sort(c, n, true, s);
+    COUNT_LAUNCH();
+    k_sorted_keys<<<grid_for(n), kThreads, 0, s>>>(n, c->skey.p, c->key.p, c->orig_key.p,
+                                                   c->d_small, c->dup_list.p, dupcap);
+  }
   int32_t* vin = c->sval.p;
-  COUNT_LAUNCH();
-  k_sorted_keys<<<grid_for(n), kThreads, 0, s>>>(n, kin, c->key.p, c->orig_key.p, c->d_small,
-                                                 c->dup_list.p, dupcap);
   // equal keys in the reference's order (an empty launch when there are none),
   // before the duplicate fix shifts them: the replay rewrites the sorted
   // indices, which the gather below then follows
@@ -1440,7 +1678,7 @@ int sort_keys_device(Ctx* c, int64_t n, const int64_t* d_in, int64_t* d_kout, in
   const int64_t nblk_sort = (n + kSortChunk - 1) / kSortChunk;
   if (!ensure(c, c->skey, n, "skey") || !ensure(c, c->skey_alt, n, "skey_alt") ||
       !ensure(c, c->sval, n, "sval") || !ensure(c, c->sval_alt, n, "sval_alt") ||
-      !ensure(c, c->hist, kMaxDigits * nblk_sort + 1, "hist") ||
+      !ensure(c, c->hist, std::max<int64_t>(kMaxDigits * nblk_sort, kMaxDigits * kCoopTiles) + 1, "hist") ||
       !ensure(c, c->scan_tmp, 2 * ((kMaxDigits * nblk_sort + n) / 2048 + 64), "scan_tmp") ||
       !ensure(c, c->cstart, n, "cstart") || !ensure(c, c->cend, n, "cend") ||
       !ensure(c, c->sstart, n, "sstart") || !ensure(c, c->send, n, "send") ||
@@ -1448,11 +1686,12 @@ int sort_keys_device(Ctx* c, int64_t n, const int64_t* d_in, int64_t* d_kout, in
     return PEPCG_ERR_OOM;
   unsigned long long* npair = c->d_small + 11;
   if (!cuda_ok(c, cudaMemsetAsync(c->d_status, 0, sizeof(uint32_t), s), "memset status") ||
-      !cuda_ok(c, cudaMemsetAsync(npair, 0, sizeof(unsigned long long), s), "memset"))
+      !cuda_ok(c, cudaMemsetAsync(npair, 0, sizeof(unsigned long long), s), "memset") ||
+      !cuda_ok(c, cudaMemsetAsync(c->barrier_word(0), 0, sizeof(unsigned), s), "memset"))
     return PEPCG_ERR_CUDA;
   COUNT_LAUNCH();
   k_sortkeys_load<<<grid_for(n), kThreads, 0, s>>>(n, d_in, c->skey.p, c->sval.p);
-  lsd_sort(c, n, false, s);
+  if (!coop_sort<false>(c, n, 0, s)) lsd_sort(c, n, false, s);
   count_pairs_launch(n, c->skey.p, npair, s);
   if (!tie_order_launch(c, tie_args(c, n, npair), s)) return PEPCG_ERR_CUDA;
   COUNT_LAUNCH();

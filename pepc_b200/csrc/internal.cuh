@@ -88,6 +88,33 @@ __device__ __forceinline__ void st256f(void* p, float4 a, float4 b) {
                "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w) : "memory");
 }
 
+// Barrier over the blocks of a cooperative launch (every block resident at
+// once): the caller counts the barriers, target = barriers so far x blocks, on a
+// word that was zero at the launch.  Writes before it are visible after it to
+// plain loads (never ld.global.nc) of every block: thread 0's fences order the block's
+// accesses on both sides, as cooperative_groups' grid.sync does.  The wait is
+// bounded (seconds): if it runs out the status word gets ST_TIMEOUT and every
+// thread of the block sees false and returns.
+constexpr unsigned kBarrierTries = 1u << 22;
+__device__ __forceinline__ bool grid_barrier(unsigned* word, unsigned target, uint32_t* status) {
+  __syncthreads();
+  int late = 0;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(word, 1u);
+    unsigned seen = 0, tries = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(word) : "memory");
+    } while (seen < target && ++tries < kBarrierTries);
+    if (seen < target) {
+      late = 1;
+      atomicOr(status, ST_TIMEOUT);
+    }
+    __threadfence();
+  }
+  return __syncthreads_or(late) == 0;
+}
+
 // The upward pass's level-ordered copy of a node: centre and charge,
 // (abs_charge, bmax), and the links by which the 64-target group walk
 // traverses the tree in this order (a twig's children are consecutive here):
@@ -171,7 +198,8 @@ struct Ctx {
   uint32_t* d_status = nullptr;
   unsigned long long* d_small = nullptr;  // [0] dup count, [1] nnodes, [2] tile count, ...
                                           // [8], [9] walk bucket queues (one per walk
-                                          // stream), [10] adjoint item queue
+                                          // stream), [10] adjoint item queue,
+                                          // [16], [17] grid barriers
   double box[9];
   double boxlength2[kMaxLevel + 1];
   int max_level = 0;
@@ -244,6 +272,8 @@ struct Ctx {
   // Slot 0 serves walks on the context stream, slot 1 walks on walk2.
   unsigned int* walk_queue(int slot = 0) { return reinterpret_cast<unsigned int*>(d_small + 8 + slot); }
   unsigned long long* item_queue() { return d_small + 10; }
+  // counting words of the cooperative kernels' barriers, zeroed before each launch
+  unsigned int* barrier_word(int k) { return reinterpret_cast<unsigned int*>(d_small + 16) + k; }
 };
 
 // The lanes of one pack of the packed per-tile walks: pack b holds the whole
