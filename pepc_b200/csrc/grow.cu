@@ -1170,35 +1170,286 @@ __global__ void __launch_bounds__(256) k_level_scatter(int64_t M, const int2* __
 
 // Upward pass: tree_node_update_from_children / shift_multipoles_up
 // (module_tree_grow.f90:762-821, coulomb/module_interaction_specific.f90:84-140),
-// level-synchronous: one launch per level, deepest first; every child of a
-// level-L twig was finished by an earlier launch, so there are no fences and
-// no atomics.  One thread per twig, in the level's RPO order; every sum runs
-// over the children in key order (child slot k = nc-1 .. 0, slot 0 being the
-// last child) with the reference's operations in its order (no contraction:
-// this file is compiled with --fmad=false).
+// level-synchronous, deepest level first; every child of a level-L twig was
+// finished before, so there are no atomics.  Every sum runs over the children in
+// key order (child slot k = nc-1 .. 0, slot 0 being the last child) with the
+// reference's operations in its order (no contraction: this file is compiled with
+// --fmad=false).
 //
-// Memory: a twig's own data (twig list, tinfo, scanned counts) is read at
-// its list position; its children's records from the level-ordered copy
-// (drec: consecutive threads read consecutive runs), and its twig children's
-// nine moments from dmom at their twig-list positions (kDmomStride doubles
-// each), likewise consecutive for consecutive parents.  The kernel is bound by
-// its count of scattered memory instructions (each warp load touches ~10
-// sectors), so the children are read in two passes (the sums that give the
-// centre, then the shifted moments; the second pass re-reads from L1 rather
-// than holding eight records in registers), centres as single 256-bit loads.
-// The twig writes its record both to the RPO arrays the walks read (nc4, mom,
-// mom32: whole sectors, 256-bit stores) and to the level-ordered copy its
-// parent will read.
+// Eight lanes per twig.  Lane k reads child k: its level-ordered record (drec: a
+// twig's children are one run) and, a twig child's, its nine moments (dmom at
+// their twig-list positions, one run too), all in one round.  The children's
+// addends go through shared memory, and each lane runs one of the sums over
+// them in order; the centre comes first (eight sums: charge, |charge|, both centre
+// candidates), then the shifted moments (27 addends per child in nine sums, and
+// bmax).  The results are stored by pieces of 16 or 32 bytes, a piece per lane: to
+// the RPO arrays the walks read (nc4, mom, mom32) and the level-ordered copy.
+// With one thread per twig the loads were scattered (about ten sectors per
+// request), and the 216 dependent additions of a full twig one thread's chain; wide
+// levels, which have threads enough to hide both, keep that form (k_upward_wide).
 constexpr int kUpThreads = 128;
+constexpr int kUpRow = 9;    // a row of eight addends, padded
+constexpr int kUpRows = 28;
 
-__global__ void __launch_bounds__(kUpThreads) k_upward_level(
-    int level, const int32_t* __restrict__ lvl, const int32_t* __restrict__ twiglist,
-    const int2* __restrict__ tinfo, const int32_t* __restrict__ cfirst,
-    const int32_t* __restrict__ tfirst, const int32_t* __restrict__ nleaves,
-    LevelRecord* __restrict__ drec, double* __restrict__ dmom, double4* __restrict__ nc4,
-    double* __restrict__ mom, float4* __restrict__ mom32) {
-  const int cnt = lvl[level];
-  const int base = level_base(lvl, level);
+struct UpArgs {
+  const int32_t* lvl;
+  const int32_t* twiglist;
+  const int2* tinfo;
+  const int32_t* cfirst;
+  const int32_t* tfirst;
+  const int32_t* nleaves;
+  LevelRecord* drec;
+  double* dmom;
+  double4* nc4;
+  double* mom;
+  float4* mom32;
+};
+
+// ld256 that stays where it is written: for records that the running kernel wrote
+// before a barrier
+__device__ __forceinline__ double4 ld256_ordered(const void* p) {
+  double4 v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
+// v + the rows r .. r + nr - 1 of each child, the children in key order
+__device__ __forceinline__ double child_sum(const double* T, int r, int nr, int nc) {
+  double v = 0.0;
+#pragma unroll
+  for (int k = 7; k >= 0; --k)
+    if (k < nc) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < nr) v = v + T[(r + j) * kUpRow + k];
+    }
+  return v;
+}
+
+// what a twig's list entry holds (fixed before the upward pass)
+struct TwigHead {
+  int P;          // position in the twig list, -1: none
+  int32_t u, nlv;
+  int2 ti;
+  int cs, ts;     // level-order position of child slot 0, list position of the first twig child
+};
+__device__ __forceinline__ TwigHead twig_head(const UpArgs& A, int P, bool on) {
+  TwigHead h{-1, 0, 0, make_int2(0, 0), 0, 0};
+  if (on) {
+    h.P = P;
+    h.u = __ldg(A.twiglist + P);
+    h.ti = __ldg(A.tinfo + P);
+    h.cs = __ldg(A.cfirst + P) + 1;
+    h.ts = __ldg(A.tfirst + P) + 1;
+    h.nlv = __ldg(A.nleaves + h.u);
+  }
+  return h;
+}
+
+// the twig of head h by this group of eight lanes; T: the group's kUpRows rows.
+// Called by whole warps.
+__device__ __forceinline__ void upward_twig(const UpArgs& A, int level, const TwigHead& h, double* T) {
+  const int c = threadIdx.x & 7;
+  const bool on = h.P >= 0;
+  const int64_t u = h.u;
+  const int nc = h.ti.x & 0xff, pu = h.ti.y, cs = h.cs, ts = h.ts, P = h.P;
+  const int32_t nlv = h.nlv;
+  double4 a = make_double4(0.0, 0.0, 0.0, 0.0);
+  double2 ab = make_double2(0.0, 0.0);
+  double m[10];
+#pragma unroll
+  for (int j = 0; j < 10; ++j) m[j] = 0.0;
+  if (on) {
+    const int2 ti = h.ti;
+    if (c < nc) {
+      const unsigned lm = (unsigned)ti.x >> 8;  // leaf children, by slot
+      const LevelRecord* rc = A.drec + cs + c;
+      a = ld256_ordered(&rc->pos);
+      ab = rc->ab;
+      if (!((lm >> c) & 1u)) {
+        const double2* src = reinterpret_cast<const double2*>(
+            A.dmom + kDmomStride * (int64_t)(ts + __popc(~lm & ((1u << c) - 1u))));
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+          const double2 v = src[j];
+          m[2 * j] = v.x;
+          m[2 * j + 1] = v.y;
+        }
+      }
+      T[c] = a.w;
+      T[kUpRow + c] = ab.x;
+      T[2 * kUpRow + c] = a.x * ab.x;
+      T[3 * kUpRow + c] = a.y * ab.x;
+      T[4 * kUpRow + c] = a.z * ab.x;
+      T[5 * kUpRow + c] = a.x;
+      T[6 * kUpRow + c] = a.y;
+      T[7 * kUpRow + c] = a.z;
+    }
+  }
+  __syncwarp();
+  const double s = child_sum(T, c, 1, nc);
+  const double charge = __shfl_sync(0xffffffffu, s, 0, 8);
+  const double absq = __shfl_sync(0xffffffffu, s, 1, 8);
+  // the centre: abs_charge-weighted (sums 2..4), or the plain mean when the
+  // |charge| sum is 0 (sums 5..7)
+  const double ctr = s / (absq != 0.0 ? absq : (double)nc);
+  const int o = absq != 0.0 ? 2 : 5;
+  const double cx = __shfl_sync(0xffffffffu, ctr, o, 8);
+  const double cy = __shfl_sync(0xffffffffu, ctr, o + 1, 8);
+  const double cz = __shfl_sync(0xffffffffu, ctr, o + 2, 8);
+  __syncwarp();
+  if (c < nc) {
+    const double s0 = cx - a.x, s1 = cy - a.y, s2 = cz - a.z;
+    const double q = a.w;
+    double* t = T + c;
+    t[0] = m[0];
+    t[1 * kUpRow] = q * s0;
+    t[2 * kUpRow] = m[1];
+    t[3 * kUpRow] = q * s1;
+    t[4 * kUpRow] = m[2];
+    t[5 * kUpRow] = q * s2;
+    t[6 * kUpRow] = m[3];
+    t[7 * kUpRow] = m[0] * s0;
+    t[8 * kUpRow] = (0.5 * q) * (s0 * s0);
+    t[9 * kUpRow] = m[4];
+    t[10 * kUpRow] = m[1] * s1;
+    t[11 * kUpRow] = (0.5 * q) * (s1 * s1);
+    t[12 * kUpRow] = m[5];
+    t[13 * kUpRow] = m[2] * s2;
+    t[14 * kUpRow] = (0.5 * q) * (s2 * s2);
+    t[15 * kUpRow] = m[6];
+    t[16 * kUpRow] = m[0] * s1;
+    t[17 * kUpRow] = m[1] * s0;
+    t[18 * kUpRow] = (q * s0) * s1;
+    t[19 * kUpRow] = m[7];
+    t[20 * kUpRow] = m[1] * s2;
+    t[21 * kUpRow] = m[2] * s1;
+    t[22 * kUpRow] = (q * s1) * s2;
+    t[23 * kUpRow] = m[8];
+    t[24 * kUpRow] = m[2] * s0;
+    t[25 * kUpRow] = m[0] * s2;
+    t[26 * kUpRow] = (q * s2) * s0;
+    t[27 * kUpRow] = sqrt((s0 * s0 + s1 * s1) + s2 * s2) + ab.y;
+  }
+  __syncwarp();
+  // lane: sums of rows r .. r + nr - 1, result slot (the order of mom); lanes 1 and 2
+  // run two short ones
+  //   0: zx   1: d0, d1   2: d2, bmax   3, 4, 5: q0, q1, q2   6: xy   7: yz
+  const int r = c == 0 ? 23 : c < 3 ? 4 * (c - 1) : c < 6 ? 6 + 3 * (c - 3) : 15 + 4 * (c - 6);
+  const int nr = c == 1 || c == 2 ? 2 : c >= 3 && c < 6 ? 3 : 4;
+  const double v0 = child_sum(T, r, nr, nc);
+  double v1 = 0.0;
+  if (c == 1) v1 = child_sum(T, 2, 2, nc);
+  if (c == 2) {
+#pragma unroll
+    for (int k = 7; k >= 0; --k)
+      if (k < nc) {
+        const double v = T[27 * kUpRow + k];
+        if (k == nc - 1 || v > v1) v1 = v;
+      }
+  }
+  __syncwarp();
+  T[c == 0 ? 8 : c == 1 ? 0 : c] = v0;  // d0 d1 d2 q0 q1 q2 xy yz zx absq bmax 0
+  if (c == 1) T[1] = v1;
+  if (c == 2) T[10] = v1;
+  if (c == 3) T[9] = absq;
+  if (c == 4) T[11] = 0.0;
+  __syncwarp();
+  if (on) {
+    LevelRecord* rp = A.drec + pu;
+    if (c == 0) {
+      st256(A.nc4 + u, make_double4(cx, cy, cz, charge));
+    } else if (c == 1) {
+      st256(&rp->pos, make_double4(cx, cy, cz, charge));
+    } else if (c == 2) {
+      st256(&rp->ab, make_double4(absq, T[10], __hiloint2double(level | (nc << 16), cs),
+                                  __hiloint2double((int)u, nlv)));
+    } else if (c < 6) {
+      const double* t = T + 4 * (c - 3);
+      st256(A.mom + kMomStride * u + 4 * (c - 3), make_double4(t[0], t[1], t[2], t[3]));
+    } else if (c == 6) {
+      // FP32 copy for the mixed walk, the quadrupole matrix M (off-diagonals
+      // halved) scaled by 3: (px, py, pz, 3qxx), (3qyy, 3qzz, 1.5qxy, 1.5qyz),
+      // (1.5qzx, qxx+qyy+qzz, charge, 0), padded to a whole 64-byte record
+      st256f(A.mom32 + kMom32Stride * u,
+             make_float4((float)T[0], (float)T[1], (float)T[2], (float)(3.0 * T[3])),
+             make_float4((float)(3.0 * T[4]), (float)(3.0 * T[5]), (float)(1.5 * T[6]),
+                         (float)(1.5 * T[7])));
+    } else {
+      st256f(A.mom32 + kMom32Stride * u + 2,
+             make_float4((float)(1.5 * T[8]), (float)((T[3] + T[4]) + T[5]), (float)charge, 0.f),
+             make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    if (c < 5)
+      reinterpret_cast<double2*>(A.dmom + kDmomStride * (int64_t)P)[c] =
+          make_double2(T[2 * c], c == 4 ? 0.0 : T[2 * c + 1]);
+  }
+  __syncwarp();
+}
+
+__global__ void __launch_bounds__(kUpThreads) k_upward_level(int level, UpArgs A) {
+  __shared__ double s_t[kUpThreads / 8 * kUpRows * kUpRow];
+  double* T = s_t + (threadIdx.x >> 3) * (kUpRows * kUpRow);
+  const int cnt = A.lvl[level];
+  const int base = level_base(A.lvl, level);
+  for (int i0 = blockIdx.x * (kUpThreads / 8); i0 < cnt; i0 += gridDim.x * (kUpThreads / 8)) {
+    const int i = i0 + (threadIdx.x >> 3);
+    upward_twig(A, level, twig_head(A, base + i, i < cnt), T);
+  }
+}
+
+// All levels in one cooperative launch, a grid barrier between them; the list
+// entries of a block's first twigs of the next level are read before it.
+__global__ void __launch_bounds__(kUpThreads) k_upward_all(int top, UpArgs A, unsigned* word,
+                                                          uint32_t* status) {
+  __shared__ double s_t[kUpThreads / 8 * kUpRows * kUpRow];
+  __shared__ int s_cnt[kMaxLevel + 1], s_base[kMaxLevel + 1];
+  double* T = s_t + (threadIdx.x >> 3) * (kUpRows * kUpRow);
+  if (threadIdx.x <= kMaxLevel) {
+    s_cnt[threadIdx.x] = A.lvl[threadIdx.x];
+    s_base[threadIdx.x] = level_base(A.lvl, threadIdx.x);
+  }
+  __syncthreads();
+  const int step = gridDim.x * (kUpThreads / 8);
+  const int first = blockIdx.x * (kUpThreads / 8) + (threadIdx.x >> 3);
+  unsigned barriers = 0;
+  TwigHead h = twig_head(A, s_base[top] + first, first < s_cnt[top]);
+  for (int level = top; level >= 0; --level) {
+    const int cnt = s_cnt[level], base = s_base[level];
+    for (int i0 = blockIdx.x * (kUpThreads / 8), i = first; i0 < cnt; i0 += step, i += step) {
+      if (i != first) h = twig_head(A, base + i, i < cnt);
+      upward_twig(A, level, h, T);
+    }
+    if (level > 0) {
+      h = twig_head(A, s_base[level - 1] + first, first < s_cnt[level - 1]);
+      if (gridDim.x > 1) {
+        if (!grid_barrier(word, ++barriers * gridDim.x, status)) return;
+      } else {
+        __syncthreads();
+      }
+    }
+  }
+}
+
+// One thread per twig, for wide levels: the kernel is bound by its count of
+// scattered memory instructions (each warp load touches ~10 sectors), so the
+// children are read in two passes (the sums that give the centre, then the shifted
+// moments; the second pass re-reads from L1 rather than holding eight records in
+// registers), centres as single 256-bit loads.
+__global__ void __launch_bounds__(kUpThreads) k_upward_wide(int level, UpArgs A) {
+  const int32_t* __restrict__ twiglist = A.twiglist;
+  const int2* __restrict__ tinfo = A.tinfo;
+  const int32_t* __restrict__ cfirst = A.cfirst;
+  const int32_t* __restrict__ tfirst = A.tfirst;
+  const int32_t* __restrict__ nleaves = A.nleaves;
+  LevelRecord* __restrict__ drec = A.drec;
+  double* __restrict__ dmom = A.dmom;
+  double4* __restrict__ nc4 = A.nc4;
+  double* __restrict__ mom = A.mom;
+  float4* __restrict__ mom32 = A.mom32;
+  const int cnt = A.lvl[level];
+  const int base = level_base(A.lvl, level);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
     const int P = base + i;
     const int64_t u = twiglist[P];
@@ -1461,6 +1712,47 @@ static TieArgs tie_args(Ctx* c, int64_t n, const unsigned long long* ndup) {
   return a;
 }
 
+// The upward pass: one cooperative launch where the widest level leaves the chip
+// short of work, else a launch per level, wide levels with one thread per twig.
+// Whole phase, us, a launch per level and one thread per twig -> this (eight lanes
+// with a launch per level in brackets): 1,000 particles 101 -> 62 (83), 16,411: 146 ->
+// 80 (103), 100,003: 168 -> 109 (122), 200,003 (widest level 33,000): 195 -> 138 (152);
+// from there a launch per level is as good (300,000: 163 against 162), and for 4M,
+// eight lanes on the levels below 30,000 twigs only: 702 -> 667 (all levels: 978).
+// Past 296 blocks the barriers cost more than they bring until a level has twigs for all
+// (60,013: 97 against 101 with 592; 200,003: 148 against 138).
+constexpr int kUpFusedWidest = 40000;
+constexpr int kUpWide = 30000;
+static void upward_pass(Ctx* c, const UpArgs& U, cudaStream_t s) {
+  int64_t widest = 0;
+  for (int L = 0; L <= kMaxLevel; ++L) widest = std::max<int64_t>(widest, c->lvl_host[L]);
+  if (widest <= kUpFusedWidest) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)std::min<int64_t>((widest + kUpThreads / 8 - 1) / (kUpThreads / 8),
+                                                   widest > 16384 ? 592 : 296));
+    cfg.blockDim = dim3(kUpThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_upward_all, c->max_level - 1, U, c->barrier_word(1), c->d_status) ==
+        cudaSuccess) {
+      COUNT_LAUNCH();
+      return;
+    }
+    cudaGetLastError();  // level by level instead
+  }
+  for (int L = c->max_level - 1; L >= 0; --L) {
+    const int64_t cnt = c->lvl_host[L];
+    if (cnt <= 0) continue;
+    COUNT_LAUNCH();
+    if (cnt >= kUpWide) k_upward_wide<<<grid_for(cnt, kUpThreads), kUpThreads, 0, s>>>(L, U);
+    else k_upward_level<<<grid_for(cnt, kUpThreads / 8), kUpThreads, 0, s>>>(L, U);
+  }
+}
+
 int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const double* dz,
                 const double* dq, cudaEvent_t q_ready) {
   cudaStream_t s = c->stream;
@@ -1624,15 +1916,9 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
                                             c->nc4.p, c->drec.p, c->lvlpos.p, c->child8.p,
                                             c->nchild.p, c->tinfo.p, cc, tcn);
     exclusive_scan2<int32_t>(cc, cc, tcn, tcn, ntw, c->scan_tmp.p, s);
-    float4* m32 = reinterpret_cast<float4*>(c->mom32.p);
-    for (int L = c->max_level - 1; L >= 0; --L) {
-      const int64_t cnt = c->lvl_host[L];
-      if (cnt <= 0) continue;
-      COUNT_LAUNCH();
-      k_upward_level<<<grid_for(cnt, kUpThreads), kUpThreads, 0, s>>>(
-          L, c->lvlcnt.p, c->twiglist.p, c->tinfo.p, cc, tcn, c->nleaves.p, c->drec.p, c->dmom.p, c->nc4.p,
-          c->mom.p, m32);
-    }
+    UpArgs U{c->lvlcnt.p, c->twiglist.p, c->tinfo.p, cc, tcn, c->nleaves.p, c->drec.p,
+             c->dmom.p, c->nc4.p, c->mom.p, reinterpret_cast<float4*>(c->mom32.p)};
+    upward_pass(c, U, s);
   }
   cudaEventRecord(c->ev[4], s);
   if (!cuda_ok(c, cudaGetLastError(), "grow kernels")) return PEPCG_ERR_CUDA;
