@@ -394,7 +394,7 @@ int pepcg_destroy(void* ctx) {
   release(c->parent); release(c->nchild); release(c->twiglist); release(c->lvlcnt); release(c->lvlblk);
   release(c->drec); release(c->lvlpos); release(c->dmom);
   release(c->tinfo); release(c->tcounts); release(c->macb); release(c->first_part);
-  release(c->nleaves); release(c->child8); release(c->wstack); release(c->leafnode);
+  release(c->nleaves); release(c->child8); release(c->wstack); release(c->over); release(c->leafnode);
   release(c->adj); release(c->fpo2rpo); release(c->rpo2fpo); release(c->nkey);
   release(c->tiles); release(c->counters); release(c->tgt); release(c->tkeys);
   for (void* p : {(void*)c->d_box, (void*)c->d_status, (void*)c->d_small, (void*)c->d_vbox,

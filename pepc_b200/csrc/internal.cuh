@@ -183,7 +183,8 @@ struct Ctx {
   DBuf<double> macb;       // per-twig MAC threshold for mac_select != 0
   int32_t lvl_host[kMaxLevel + 1] = {0};  // twigs per level of the grown tree
   DBuf<int4> child8;  // up to 8 children (RPO indices) per twig, as 2 x int4
-  DBuf<int32_t> wstack;  // per-warp traversal stacks of the wide group walk
+  DBuf<int32_t> wstack;  // traversal stacks of the group walks (per warp or block) and list walks
+  DBuf<int32_t> over;    // list walks: buckets whose lists did not fit
   DBuf<int32_t> leafnode;  // key-ordered particle -> RPO index of its leaf
   DBuf<double> adj;        // adjoint records, 16 doubles per node
   DBuf<int32_t> fpo2rpo, rpo2fpo;

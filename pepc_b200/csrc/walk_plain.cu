@@ -63,6 +63,14 @@ struct WalkArgs {
   // spatial_interaction_cutoff (module_mirror_boxes.f90:52), when finite
   int has_cut;
   double cut[3];
+  // list walk (k_walk_list64)
+  const LevelRecord* drec;
+  const int32_t* rpo2fpo;
+  const int32_t* fpo2rpo;
+  uint2* lstack;       // kListStack entries per resident block
+  // buckets (packs) whose lists did not fit: [0] their number, then their indices.
+  // Written by k_walk_list64; k_walk_target64 / k_walk_tilepack64 walk them (kOnly)
+  int32_t* over;
 };
 
 // any(abs(delta) >= spatial_interaction_cutoff) (module_tree_walk_pthreads.f90:
@@ -88,7 +96,9 @@ __device__ __forceinline__ void warp_add_counters(unsigned long long* ctr, unsig
   }
 }
 
-template <int kLaw, bool kCut>
+// kOnly: walks the buckets that A.over lists (a separate instantiation: the test inside
+// the queue loop cost the walk of 250,000 targets 10 %)
+template <int kLaw, bool kCut, bool kOnly = false>
 __global__ void __launch_bounds__(kWalkThreads) k_walk_target64(WalkArgs A) {
   __shared__ double s_bl2[kMaxLevel + 1];
   __shared__ double s_vb[3 * 125];
@@ -102,6 +112,10 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_target64(WalkArgs A) {
     unsigned b = 0;
     if (lane == 0) b = atomicAdd(A.queue, 1u);
     b = __shfl_sync(0xffffffffu, b, 0);
+    if constexpr (kOnly) {
+      if ((int)b >= A.over[0]) break;
+      b = (unsigned)A.over[1 + b];
+    }
     if ((int64_t)b * 32 >= A.nt) break;
     const int64_t t = (int64_t)b * 32 + lane;
     const bool valid = t < A.nt;
@@ -306,7 +320,7 @@ __global__ void __launch_bounds__(kWalkThreads, kTPL == 1 ? 6 : 4) k_walk_tile64
 // decides accept / open by a ballot over its own lanes.  A lane's sequence of
 // interactions is exactly its tile's, so fields, work and MAC counts equal
 // the one-tile-per-warp walk's.
-template <int kLaw, bool kCut>
+template <int kLaw, bool kCut, bool kOnly = false>
 // Six resident blocks per SM (80 registers, a few spilled): at 4M, T = 16,
 // 260 ms against 296 ms at the unbounded 110 registers (four blocks).
 __global__ void __launch_bounds__(kWalkThreads, 6) k_walk_tilepack64(WalkArgs A) {
@@ -323,6 +337,10 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_walk_tilepack64(WalkArgs A)
     unsigned b = 0;
     if (lane == 0) b = atomicAdd(A.queue, 1u);
     b = __shfl_sync(0xffffffffu, b, 0);
+    if constexpr (kOnly) {
+      if ((int)b >= A.over[0]) break;
+      b = (unsigned)A.over[1 + b];
+    }
     if ((int64_t)b >= npk) break;
     int tl0, len;
     const int64_t t0 = A.pstart[b];
@@ -406,6 +424,300 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_walk_tilepack64(WalkArgs A)
       A.ex[t] = e0; A.ey[t] = e1; A.ez[t] = e2; A.pot[t] = ph; A.work[t] = w;
     }
     if (__any_sync(0xffffffffu, !complete) && lane == 0) atomicOr(A.status, ST_INCOMPLETE);
+  }
+  warp_add_counters(A.counters, c_leaf, c_twig, c_mac);
+}
+
+// ---------------------------------------------------------------------------
+// The same two walks (law 3, no cutoff, one box) by one block per bucket of 32
+// targets or pack of tiles, bit for bit: a target's result is the sum of its
+// interactions' terms in the order of the walk, and that order is the node order
+// (RPO for the per-target walk, forward preorder for tiles).  So the interactions can be
+// found and evaluated in any order, as long as each target's terms are added in
+// node order:
+//  1. the block finds the bucket's interactions from a shared stack of (node, targets that
+//     reach it), eight nodes per warp and round, lane = target; a node's accepting targets
+//     give one list entry (order index, leaf flag, target mask), the others open it;
+//  2. the list is sorted by the order index;
+//  3. batches of 32 entries: the (entry, target) pairs are packed, twigs and leaves
+//     apart, so that every lane evaluates an interaction; the terms go to shared memory;
+//     then one warp per component adds them per target, entry by entry.
+// The walks above give a bucket to one warp, a serial chain of dependent loads and FP64
+// latencies (4,099 particles are 129 such warps), and evaluate with 77 % of the lanes
+// active (here 96 %).
+// Lists hold kListCap entries (shared memory: two blocks per SM); a longer
+// one is left to the walks above (A.over).
+constexpr int kListThreads = 256;
+constexpr int kListWarps = kListThreads / 32;
+constexpr int kListCap = 8192;
+constexpr int kListNodes = 8;   // nodes per warp and round
+constexpr int kListPop = kListWarps * kListNodes;
+// a pop takes at most kListPop entries and each pushes at most 8 (one level down)
+constexpr int kListStack = (kMaxLevel + 2) * 8 * kListPop;
+constexpr int kListBatch = 32;  // entries per batch
+
+struct __align__(16) ListShared {
+  unsigned long long list[kListCap];            // order index << 33 | leaf << 32 | target mask
+  double term[kListBatch][4][32];
+  uint16_t pair[2][kListBatch * 32];            // twigs, leaves: entry << 5 | target
+  double tgt[3][32];
+  double bl2[kMaxLevel + 1];
+  uint2 cnt[kListWarps];
+  unsigned partner[32];
+  uint32_t self[2][kListBatch];                 // by batch parity: targets whose own leaf the entry is
+  unsigned bucket;
+};
+
+template <bool kTile>
+__global__ void __launch_bounds__(kListThreads, 2) k_walk_list64(WalkArgs A) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  ListShared& S = *reinterpret_cast<ListShared*>(dyn);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  for (int i = tid; i <= kMaxLevel; i += kListThreads) S.bl2[i] = A.bl2[i];
+  uint2* stack = A.lstack + (int64_t)blockIdx.x * kListStack;
+  const int64_t nbk = kTile ? (int64_t)*A.npacks : (A.nt + 31) / 32;
+  const double vx = A.vbox[0], vy = A.vbox[1], vz = A.vbox[2];
+  unsigned long long c_leaf = 0, c_twig = 0, c_mac = 0;
+  for (;;) {
+    if (tid == 0) S.bucket = atomicAdd(A.queue, 1u);
+    if (tid < 32) S.partner[tid] = 0u;
+    __syncthreads();
+    const int64_t b = S.bucket;
+    if (b >= nbk) break;
+    bool valid;
+    int64_t t0;
+    unsigned tmask = 0u;  // the lanes of this lane's tile
+    if (kTile) {
+      int tl0, len;
+      t0 = A.pstart[b];
+      valid = pack_lane(A.pstart, A.tflag, b, lane, tl0, len);
+      tmask = valid ? (((len >= 32) ? 0xffffffffu : ((1u << len) - 1u)) << tl0) : 0u;
+    } else {
+      t0 = b * 32;
+      valid = t0 + lane < A.nt;
+    }
+    const unsigned all = __ballot_sync(0xffffffffu, valid);
+    if (all == 0u) {
+      if (tid == 0) atomicOr(A.status, ST_INCOMPLETE);  // a pack must start with a tile
+      __syncthreads();
+      continue;
+    }
+    const int64_t t = t0 + lane;
+    double px = 0, py = 0, pz = 0;
+    if (valid) {
+      px = A.tx[t]; py = A.ty[t]; pz = A.tz[t];
+    }
+    // x - vbox (module_tree_walk_pthreads.f90:595, module_tree_walk_simple.f90:328)
+    const double sx = px - vx, sy = py - vy, sz = pz - vz;
+    if (w == 0) {
+      S.tgt[0][lane] = sx; S.tgt[1][lane] = sy; S.tgt[2][lane] = sz;
+    }
+    // ---- 1. the interactions.  Per tile the walk starts at the root
+    // (module_tree_walk_simple.f90:286), per target with its children (:601)
+    int top, cnt = 0;
+    bool over = false;
+    {
+      const int4 lk = A.drec[0].link;
+      const int nch = min(8, lk.y >> 16);
+      if (kTile || (lk.y & kLeafFlag)) {
+        if (tid == 0) stack[0] = make_uint2(0u, all);
+        top = 1;
+      } else {
+        if (tid < nch) stack[tid] = make_uint2((unsigned)(lk.x + nch - 1 - tid), all);
+        top = nch;
+      }
+    }
+    __syncthreads();
+    unsigned partner = 0, mac = 0;
+    while (top > 0) {
+      const int take = min(top, kListPop);
+      top -= take;
+      uint2 en[kListNodes];
+      double4 pos[kListNodes];
+      int4 lk[kListNodes];
+#pragma unroll
+      for (int j = 0; j < kListNodes; ++j) {
+        const int i = w * kListNodes + j;
+        en[j] = i < take ? stack[top + i] : make_uint2(0u, 0u);
+      }
+#pragma unroll
+      for (int j = 0; j < kListNodes; ++j) {
+        const LevelRecord* r = A.drec + en[j].x;
+        pos[j] = ld256(&r->pos);
+        lk[j] = r->link;
+      }
+      // lane j keeps node j's decision
+      unsigned my_acc = 0, my_open = 0;
+      int my_first = 0, my_nch = 0, my_rpo = 0, my_leaf = 0;
+#pragma unroll
+      for (int j = 0; j < kListNodes; ++j) {
+        const unsigned reach = en[j].y;  // 0: no node
+        const bool in = (reach >> lane) & 1u;
+        const bool leaf = (lk[j].y & kLeafFlag) != 0;
+        unsigned acc = reach;
+        if (!leaf && reach) {
+          const double dx = sx - pos[j].x, dy = sy - pos[j].y, dz = sz - pos[j].z;
+          const double dist2 = (dx * dx + dy * dy) + dz * dz;
+          const bool ok = A.theta2 * dist2 > (A.macb ? A.macb[lk[j].w] : S.bl2[lk[j].y & 0xff]);
+          const unsigned fail = __ballot_sync(0xffffffffu, in && !ok);
+          if (kTile) {
+            // a tile opens a twig if any of its targets fails; MAC evaluations
+            // stop at the first (module_tree_walk_simple.f90:343-370)
+            const unsigned tf = fail & tmask;
+            if (in && lane <= (tf ? __ffs(tf) - 1 : 32)) ++mac;
+            acc = __ballot_sync(0xffffffffu, in && tf == 0u);
+          } else {
+            if (in) ++mac;
+            acc = reach & ~fail;
+          }
+        }
+        if ((acc >> lane) & 1u) partner += leaf ? 1u : (unsigned)lk[j].z;
+        if (lane == j) {
+          my_acc = acc;
+          my_open = reach & ~acc;
+          my_first = lk[j].x;
+          my_nch = min(8, lk[j].y >> 16);
+          my_rpo = lk[j].w;
+          my_leaf = leaf ? 1 : 0;
+        }
+      }
+      const unsigned ab = __ballot_sync(0xffffffffu, my_acc != 0u);
+      const int npush = my_open ? my_nch : 0;
+      int off = npush;  // inclusive over the first kListNodes lanes
+#pragma unroll
+      for (int o = 1; o < kListNodes; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, off, o);
+        if (lane >= o) off += y;
+      }
+      const int wtotal = __shfl_sync(0xffffffffu, off, kListNodes - 1);
+      off -= npush;
+      if (lane == 0) S.cnt[w] = make_uint2((unsigned)__popc(ab), (unsigned)wtotal);
+      __syncthreads();  // the counts are in; every warp has read its stack entries
+      const uint2 c = lane < kListWarps ? S.cnt[lane] : make_uint2(0u, 0u);
+      const int lpre = (int)__reduce_add_sync(0xffffffffu, lane < w ? c.x : 0u);
+      const int ltot = (int)__reduce_add_sync(0xffffffffu, c.x);
+      off += (int)__reduce_add_sync(0xffffffffu, lane < w ? c.y : 0u);
+      const int ptot = (int)__reduce_add_sync(0xffffffffu, c.y);
+      if (cnt + ltot > kListCap || top + ptot > kListStack) {
+        over = true;
+        break;
+      }
+      if (my_acc) {
+        const unsigned idx = (unsigned)(kTile ? A.rpo2fpo[my_rpo] : my_rpo);
+        S.list[cnt + lpre + __popc(ab & lt)] =
+            ((unsigned long long)(idx << 1 | (unsigned)my_leaf) << 32) | my_acc;
+      }
+      for (int k = 0; k < npush; ++k) stack[top + off + k] = make_uint2((unsigned)(my_first + k), my_open);
+      cnt += ltot;
+      top += ptot;
+      __syncthreads();
+    }
+    if (over) {
+      if (tid == 0) A.over[1 + atomicAdd(A.over, 1)] = (int32_t)b;
+      __syncthreads();
+      continue;
+    }
+    c_mac += mac;
+    atomicAdd(&S.partner[lane], partner);
+    // ---- 2. node order: bitonic sort, padded to a power of two
+    int P = 64;
+    while (P < cnt) P <<= 1;
+    for (int i = cnt + tid; i < P; i += kListThreads) S.list[i] = ~0ull;
+    __syncthreads();
+    for (int k = 2; k <= P; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int i = tid; i < (P >> 1); i += kListThreads) {
+          const int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1)), hi = lo | j;
+          const unsigned long long x = S.list[lo], y = S.list[hi];
+          if ((x > y) == ((lo & k) == 0)) {
+            S.list[lo] = y;
+            S.list[hi] = x;
+          }
+        }
+        __syncthreads();
+      }
+    // ---- 3. terms and ordered sums: warps 0..3 add ex, ey, ez, phi, warp 4 work
+    double* const out = w == 0 ? A.ex : w == 1 ? A.ey : w == 2 ? A.ez : w == 3 ? A.pot : A.work;
+    double sum = 0.0;
+    if (w < 5 && valid) sum = out[t];
+    int par = 0;
+    for (int e0 = 0; e0 < cnt; e0 += kListBatch, par ^= 1) {
+      const int ne = min(kListBatch, cnt - e0);
+      // pairs: prefix over the batch's entries, then each warp lists four of them
+      const unsigned long long en = lane < ne ? S.list[e0 + lane] : 0ull;
+      const bool leaf = (en >> 32) & 1u;
+      const int nt = leaf ? 0 : __popc((unsigned)en), nl = leaf ? __popc((unsigned)en) : 0;
+      int both = nt | (nl << 16);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, both, o);
+        if (lane >= o) both += y;
+      }
+      const int total = __shfl_sync(0xffffffffu, both, 31);
+      const int pt = total & 0xffff, pl = total >> 16;
+      both -= nt | (nl << 16);
+#pragma unroll
+      for (int j = 0; j < kListBatch / kListWarps; ++j) {
+        const int e = w * (kListBatch / kListWarps) + j;
+        const unsigned m = __shfl_sync(0xffffffffu, (unsigned)en, e);
+        const int lf = __shfl_sync(0xffffffffu, leaf ? 1 : 0, e);
+        const int p0 = __shfl_sync(0xffffffffu, both, e);
+        if ((m >> lane) & 1u)
+          S.pair[lf][(lf ? p0 >> 16 : p0 & 0xffff) + __popc(m & lt)] = (uint16_t)(e << 5 | lane);
+        if (lane == 0) S.self[par][e] = 0u;
+      }
+      __syncthreads();  // the pairs are listed, and the last batch's terms are added
+      for (int i = tid; i < pt; i += kListThreads) {
+        const int pr = S.pair[0][i], e = pr >> 5, q = pr & 31;
+        const int idx = (int)(S.list[e0 + e] >> 33);
+        const int64_t u = kTile ? A.fpo2rpo[idx] : idx;
+        const double4 a = ld256(A.nc4 + u);
+        const double* mp = A.mom + kMomStride * u;
+        const double4 m0 = ld256(mp), m1 = ld256(mp + 4);
+        const double m[9] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w, mp[8]};
+        const double dx = S.tgt[0][q] - a.x, dy = S.tgt[1][q] - a.y, dz = S.tgt[2][q] - a.z;
+        const double dist2 = (dx * dx + dy * dy) + dz * dz;
+        double fx, fy, fz, fp;
+        law_twig64<3>(a.w, m, dx, dy, dz, dist2, A.eps2, fx, fy, fz, fp);
+        S.term[e][0][q] = fx; S.term[e][1][q] = fy; S.term[e][2][q] = fz; S.term[e][3][q] = fp;
+      }
+      for (int i = tid; i < pl; i += kListThreads) {
+        const int pr = S.pair[1][i], e = pr >> 5, q = pr & 31;
+        const int idx = (int)(S.list[e0 + e] >> 33);
+        const int64_t u = kTile ? A.fpo2rpo[idx] : idx;
+        const double4 a = ld256(A.nc4 + u);
+        const double dx = S.tgt[0][q] - a.x, dy = S.tgt[1][q] - a.y, dz = S.tgt[2][q] - a.z;
+        const double dist2 = (dx * dx + dy * dy) + dz * dz;
+        if (dist2 > 0.0) {
+          double fx, fy, fz, fp;
+          law_leaf64<3>(a.w, dx, dy, dz, dist2, A.eps2, fx, fy, fz, fp);
+          S.term[e][0][q] = fx; S.term[e][1][q] = fy; S.term[e][2][q] = fz; S.term[e][3][q] = fp;
+        } else {
+          atomicOr(&S.self[par][e], 1u << q);
+        }
+      }
+      if (tid == 0) {
+        c_twig += (unsigned)pt;
+        c_leaf += (unsigned)pl;
+      }
+      __syncthreads();
+      if (w < 4) {
+#pragma unroll 8
+        for (int e = 0; e < ne; ++e) {
+          const unsigned m = (unsigned)S.list[e0 + e] & ~S.self[par][e];
+          if ((m >> lane) & 1u) sum += S.term[e][w][lane];
+        }
+      } else if (w == 4) {
+#pragma unroll 8
+        for (int e = 0; e < ne; ++e)
+          if (((unsigned)S.list[e0 + e] >> lane) & 1u) sum += 1.0;
+      }
+    }
+    if (w < 5 && valid) out[t] = sum;
+    if (w == 0 && __any_sync(0xffffffffu, valid && S.partner[lane] != (unsigned)A.npart) && lane == 0)
+      atomicOr(A.status, ST_INCOMPLETE);
+    __syncthreads();  // the list and the partner counts may be written again
   }
   warp_add_counters(A.counters, c_leaf, c_twig, c_mac);
 }
@@ -572,6 +884,26 @@ int prepare_mac(Ctx* c, const double** macb) {
   return PEPCG_OK;
 }
 
+// Whether the plain walk of nt targets goes by k_walk_list64: while its buckets are
+// fewer than the warps that the walks by warp keep resident (2,368), and where a list
+// is likely to fit (theta >= 0.35, or a tree smaller than a list).  Walk ms, by warp ->
+// by lists, per target: 1,000 particles 0.237 -> 0.082, 4,099: 0.46 -> 0.117, 16,411
+// (Plummer, theta 0.4) 3.36 -> 1.22, 40,009: 0.86 -> 0.56; per tile 4,099: 0.46 -> 0.133, 40,009:
+// 1.10 -> 0.69.  With more buckets the lists' own work (sort, packing, a
+// node per warp step in the search: 480 instructions per 32 interactions, 158 of them
+// FP64) costs more than idle lanes: 100,003: 3.04 against 3.43, 250,000: 6.4 against 9.0.
+constexpr int64_t kListTargets = 65536;
+constexpr int kListBlocks = 148 * 2;
+static bool use_list_walk(const Ctx* c, int64_t nt, bool chunked, bool packed) {
+  const pepcg_params& p = c->prm;
+  if (p.precision != PEPCG_PRECISION_PLAIN || chunked || p.force_law != 3 || has_spatial_cutoff(p) ||
+      c->nboxes != 1)
+    return false;
+  if (p.walk != PEPCG_WALK_PER_TARGET && !packed) return false;
+  if (nt > kListTargets) return false;
+  return c->nnodes <= kListCap || (p.mac_select == 0 && p.theta2 >= 0.12);
+}
+
 int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const double* tz,
                     const int64_t* tkeys, bool self, double* ex, double* ey, double* ez,
                     double* pot, double* work, const double* tq, const ChunkPlan* plan,
@@ -706,6 +1038,20 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   A.has_cut = has_spatial_cutoff(c->prm) ? 1 : 0;
   for (int k = 0; k < 3; ++k) A.cut[k] = c->prm.spatial_interaction_cutoff[k];
   const int blocks = 148 * 8;
+  const bool lists = use_list_walk(c, nt, plan != nullptr, packed);
+  if (lists) {
+    const int64_t nbk = packed ? (nt + kPackChunk - 1) / kPackChunk * kPackSlots : (nt + 31) / 32;
+    if (!ensure(c, c->wstack, (size_t)2 * kListStack * kListBlocks, "walk stacks") ||
+        !ensure(c, c->over, nbk + 1, "walk lists"))
+      return PEPCG_ERR_OOM;
+    A.drec = c->drec.p;
+    A.rpo2fpo = c->rpo2fpo.p;
+    A.fpo2rpo = c->fpo2rpo.p;
+    A.lstack = reinterpret_cast<uint2*>(c->wstack.p);
+    A.over = c->over.p;
+    if (!cuda_ok(c, cudaMemsetAsync(c->over.p, 0, sizeof(int32_t), s), "walk lists"))
+      return PEPCG_ERR_CUDA;
+  }
   // chunks alternate between the context stream and walk2, so that each
   // chunk's walk starts while the previous one finishes its last buckets
   const bool two = nchunks > 1 && c->walk2;
@@ -732,7 +1078,13 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
         COUNT_LAUNCH();
         const int law = c->prm.force_law;
         const bool cut = A.has_cut != 0;
-        if (walk == PEPCG_WALK_PER_TARGET) {
+        if (lists) {
+          auto kern = packed ? k_walk_list64<true> : k_walk_list64<false>;
+          if (!cuda_ok(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(ListShared)), "list walk"))
+            return PEPCG_ERR_CUDA;
+          kern<<<kListBlocks, kListThreads, sizeof(ListShared), sk>>>(A);
+        } else if (walk == PEPCG_WALK_PER_TARGET) {
           launch_law_cut(law, cut, [&](auto L, auto C) {
             k_walk_target64<decltype(L)::value, decltype(C)::value><<<blocks, kWalkThreads, 0, sk>>>(A);
           });
@@ -775,6 +1127,22 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   if (plan && plan->before_sync && !plan->before_sync()) return PEPCG_ERR_CUDA;
   unsigned long long ctr[4];
   uint32_t st = 0;
+  int32_t nover = 0;
+  if (lists) {
+    if (!cuda_ok(c, cudaMemcpyAsync(&nover, c->over.p, sizeof(nover), cudaMemcpyDeviceToHost, s), "walk lists") ||
+        !cuda_ok(c, cudaStreamSynchronize(s), "walk lists"))
+      return PEPCG_ERR_CUDA;
+    if (nover > 0) {  // lists that did not fit: these buckets by the warp walks
+      COUNT_LAUNCH();
+      k_reset_counter<<<1, 1, 0, s>>>(A.queue);
+      COUNT_LAUNCH();
+      if (packed) k_walk_tilepack64<3, false, true><<<blocks, kWalkThreads, 0, s>>>(A);
+      else k_walk_target64<3, false, true><<<blocks, kWalkThreads, 0, s>>>(A);
+      cudaEventRecord(c->ev[6], s);
+      cudaEventRecord(c->ev[7], s);
+      if (!cuda_ok(c, cudaGetLastError(), "walk launch")) return PEPCG_ERR_CUDA;
+    }
+  }
   if (!cuda_ok(c, cudaMemcpyAsync(ctr, c->counters.p, 4 * sizeof(unsigned long long),
                                   cudaMemcpyDeviceToHost, s), "counters") ||
       !cuda_ok(c, cudaMemcpyAsync(&st, c->d_status, 4, cudaMemcpyDeviceToHost, s), "status") ||
