@@ -460,88 +460,144 @@ __global__ void __launch_bounds__(kAdjThreads, 5) k_adj_group(AdjArgs A) {
   }
 }
 
-// transpose of shift_multipoles_up for the twigs of one level (top-down);
-// the twigs of a level come from the per-level lists built by the grow, and
-// each twig's children are read as one run of the grow's level-ordered
-// records (drec: centre and charge, abs_charge; link.w the RPO index of the
-// child's adjoint record) and its twig children's dipoles from dmom at their
-// twig-list positions -- the values of nc4 and mom, without chasing the
-// children through meta.  Children in key order, as shift_multipoles_up.
-__global__ void k_adj_down_level(int level, const int32_t* __restrict__ lvl,
-                                 const int32_t* __restrict__ twiglist,
-                                 const int2* __restrict__ tinfo,
-                                 const int32_t* __restrict__ cfirst,
-                                 const int32_t* __restrict__ tfirst,
-                                 const LevelRecord* __restrict__ drec,
-                                 const double* __restrict__ dmom, double* __restrict__ adj) {
-  int base = 0;
-  for (int l = 0; l < level; ++l) base += lvl[l];
-  const int cnt = lvl[level];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-    const int P = base + i;
-    const int64_t u = twiglist[P];
-    const int2 ti = tinfo[P];
-    const int nc = ti.x & 0xff;
-    const unsigned lm = (unsigned)ti.x >> 8;  // leaf children, by slot
-    const LevelRecord* rc = drec + cfirst[P] + 1;  // child slot 0
-    const int ts = tfirst[P] + 1;                  // twig-list position of the first twig child
-    const double4 pc = drec[ti.y].pos;
-    const double A = drec[ti.y].ab.x;
-    const double* pa = adj + kNA * (int64_t)ti.y;
-    const double Pq = pa[0];
-    const double Pp[3] = {pa[1], pa[2], pa[3]};
-    const double PQ[6] = {pa[4], pa[5], pa[6], pa[7], pa[8], pa[9]};
-    double cocbar[3] = {pa[10], pa[11], pa[12]};
-    const double PA = pa[13];
-    // first pass: everything except the centre-of-charge chain rule
-    for (int k = 0; k < nc; ++k) {
-      const double4 cc = rc[k].pos;
-      const bool leafc = (lm >> k) & 1u;
-      double pcv[3] = {0, 0, 0};
-      if (!leafc) {
-        const double* dm = dmom + kDmomStride * (int64_t)(ts + __popc(~lm & ((1u << k) - 1u)));
-        for (int j = 0; j < 3; ++j) pcv[j] = dm[j];
-      }
-      const double qc = cc.w;
-      const double sc[3] = {pc.x - cc.x, pc.y - cc.y, pc.z - cc.z};
-      double sbar[3] = {0, 0, 0};
-      for (int j = 0; j < 3; ++j) sbar[j] += Pp[j] * qc;
-      for (int j = 0; j < 3; ++j) sbar[j] += PQ[j] * (pcv[j] + qc * sc[j]);
-      sbar[0] += PQ[3] * (pcv[1] + qc * sc[1]); sbar[1] += PQ[3] * (pcv[0] + qc * sc[0]);
-      sbar[1] += PQ[4] * (pcv[2] + qc * sc[2]); sbar[2] += PQ[4] * (pcv[1] + qc * sc[1]);
-      sbar[2] += PQ[5] * (pcv[0] + qc * sc[0]); sbar[0] += PQ[5] * (pcv[2] + qc * sc[2]);
-      double* a = adj + kNA * (int64_t)(cfirst[P] + 1 + k);
-      double aq = Pq;
-      for (int j = 0; j < 3; ++j) aq += Pp[j] * sc[j] + PQ[j] * 0.5 * sc[j] * sc[j];
-      aq += PQ[3] * sc[0] * sc[1] + PQ[4] * sc[1] * sc[2] + PQ[5] * sc[2] * sc[0];
-      a[0] += aq;
-      a[1] += Pp[0] + PQ[0] * sc[0] + PQ[3] * sc[1] + PQ[5] * sc[2];
-      a[2] += Pp[1] + PQ[1] * sc[1] + PQ[3] * sc[0] + PQ[4] * sc[2];
-      a[3] += Pp[2] + PQ[2] * sc[2] + PQ[4] * sc[1] + PQ[5] * sc[0];
-      for (int s2 = 0; s2 < 6; ++s2) a[4 + s2] += PQ[s2];
-      for (int j = 0; j < 3; ++j) {
-        a[10 + j] -= sbar[j];
-        cocbar[j] += sbar[j];
-      }
-      a[13] += PA;
+// Transpose of shift_multipoles_up (top-down), eight lanes per twig, lane k child k:
+// the twigs come from the per-level lists built by the grow, and a twig's children
+// are read as one run of the grow's level-ordered records (drec: centre and
+// charge, abs_charge), its twig children's dipoles from dmom at their twig-list
+// positions, and the adjoint records in the same level order.  Every lane takes its
+// child's record once; the children's shares of the centre's adjoint are added across the
+// lanes.  With one thread per twig, which walks its children one after the other,
+// twice, a level was a long chain, and the records were read and written twice: whole
+// pass of 100,003 particles 0.49 -> 0.09 ms, 262,144 sources 0.44 -> 0.12, 4M (call)
+// 3.25 -> 2.47.
+constexpr int kDownThreads = 128;
+struct DownArgs {
+  const int32_t* lvl;
+  const int2* tinfo;
+  const int32_t* cfirst;
+  const int32_t* tfirst;
+  const LevelRecord* drec;
+  const double* dmom;
+  double* adj;
+};
+// list entry of a twig (P < 0: none)
+struct DownHead {
+  int P, cs, ts;
+  int2 ti;
+};
+__device__ __forceinline__ DownHead down_head(const DownArgs& D, int P, bool on) {
+  DownHead h{-1, 0, 0, make_int2(0, 0)};
+  if (on) {
+    h.P = P;
+    h.ti = __ldg(D.tinfo + P);
+    h.cs = __ldg(D.cfirst + P) + 1;  // child slot 0
+    h.ts = __ldg(D.tfirst + P) + 1;  // twig-list position of the first twig child
+  }
+  return h;
+}
+
+__device__ __forceinline__ void adj_down_twig(const DownArgs& D, const DownHead& h) {
+  const int k = threadIdx.x & 7;
+  const int nc = h.ti.x & 0xff;
+  const bool have = h.P >= 0 && k < nc;
+  double PQ[6] = {0, 0, 0, 0, 0, 0}, Pp[3] = {0, 0, 0}, Pq = 0.0, PA = 0.0, A = 0.0;
+  double cocbar[3] = {0, 0, 0}, sbar[3] = {0, 0, 0}, sc[3] = {0, 0, 0}, Ac = 0.0, qc = 0.0;
+  if (have) {
+    const double2* pa = reinterpret_cast<const double2*>(D.adj + kNA * (int64_t)h.ti.y);
+    const double2 p0 = pa[0], p1 = pa[1], p2 = pa[2], p3 = pa[3], p4 = pa[4], p5 = pa[5], p6 = pa[6];
+    Pq = p0.x;
+    Pp[0] = p0.y; Pp[1] = p1.x; Pp[2] = p1.y;
+    PQ[0] = p2.x; PQ[1] = p2.y; PQ[2] = p3.x; PQ[3] = p3.y; PQ[4] = p4.x; PQ[5] = p4.y;
+    cocbar[0] = p5.x; cocbar[1] = p5.y; cocbar[2] = p6.x;
+    PA = p6.y;
+    const LevelRecord* pr = D.drec + h.ti.y;
+    const double4 pc = ld256(&pr->pos);
+    A = pr->ab.x;
+    const LevelRecord* rc = D.drec + h.cs + k;
+    const double4 cc = ld256(&rc->pos);
+    Ac = rc->ab.x;
+    qc = cc.w;
+    const unsigned lm = (unsigned)h.ti.x >> 8;  // leaf children, by slot
+    double pcv[3] = {0, 0, 0};
+    if (!((lm >> k) & 1u)) {
+      const double* dm = D.dmom + kDmomStride * (int64_t)(h.ts + __popc(~lm & ((1u << k) - 1u)));
+      for (int j = 0; j < 3; ++j) pcv[j] = dm[j];
     }
-    // second pass: coc = sum coc_c A_c / A (or the plain mean when A = 0)
-    for (int k = 0; k < nc; ++k) {
-      const double4 cc = rc[k].pos;
-      double* a = adj + kNA * (int64_t)(cfirst[P] + 1 + k);
-      if (A != 0.0) {
-        const double Ac = rc[k].ab.x;  // abs_charge (a leaf's |q|)
-        const double w = Ac / A;
-        const double cv[3] = {cc.x, cc.y, cc.z};
-        const double pv[3] = {pc.x, pc.y, pc.z};
-        double g = 0.0;
-        for (int j = 0; j < 3; ++j) {
-          a[10 + j] += cocbar[j] * w;
-          g += cocbar[j] * (cv[j] - pv[j]);
-        }
-        a[13] += g / A;
+    sc[0] = pc.x - cc.x; sc[1] = pc.y - cc.y; sc[2] = pc.z - cc.z;
+    const double v[3] = {pcv[0] + qc * sc[0], pcv[1] + qc * sc[1], pcv[2] + qc * sc[2]};
+    sbar[0] = Pp[0] * qc + PQ[0] * v[0] + PQ[3] * v[1] + PQ[5] * v[2];
+    sbar[1] = Pp[1] * qc + PQ[1] * v[1] + PQ[3] * v[0] + PQ[4] * v[2];
+    sbar[2] = Pp[2] * qc + PQ[2] * v[2] + PQ[4] * v[1] + PQ[5] * v[0];
+  }
+  for (int j = 0; j < 3; ++j) {  // over the twig's children
+    double t = sbar[j];
+    for (int o = 1; o < 8; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    cocbar[j] += t;
+  }
+  if (!have) return;
+  // coc = sum coc_c A_c / A (or the plain mean when A = 0); sc is coc - coc_c
+  double cb[3], ab = PA;
+  if (A != 0.0) {
+    const double wt = Ac / A;
+    double g = 0.0;
+    for (int j = 0; j < 3; ++j) {
+      cb[j] = cocbar[j] * wt;
+      g -= cocbar[j] * sc[j];
+    }
+    ab += g / A;
+  } else {
+    for (int j = 0; j < 3; ++j) cb[j] = cocbar[j] / (double)nc;
+  }
+  double aq = Pq;
+  for (int j = 0; j < 3; ++j) aq += Pp[j] * sc[j] + PQ[j] * 0.5 * sc[j] * sc[j];
+  aq += PQ[3] * sc[0] * sc[1] + PQ[4] * sc[1] * sc[2] + PQ[5] * sc[2] * sc[0];
+  double2* a = reinterpret_cast<double2*>(D.adj + kNA * (int64_t)(h.cs + k));
+  double2 r[7];
+#pragma unroll
+  for (int j = 0; j < 7; ++j) r[j] = a[j];
+  r[0].x += aq;
+  r[0].y += Pp[0] + PQ[0] * sc[0] + PQ[3] * sc[1] + PQ[5] * sc[2];
+  r[1].x += Pp[1] + PQ[1] * sc[1] + PQ[3] * sc[0] + PQ[4] * sc[2];
+  r[1].y += Pp[2] + PQ[2] * sc[2] + PQ[4] * sc[1] + PQ[5] * sc[0];
+  r[2].x += PQ[0]; r[2].y += PQ[1]; r[3].x += PQ[2];
+  r[3].y += PQ[3]; r[4].x += PQ[4]; r[4].y += PQ[5];
+  r[5].x += cb[0] - sbar[0];
+  r[5].y += cb[1] - sbar[1];
+  r[6].x += cb[2] - sbar[2];
+  r[6].y += ab;
+#pragma unroll
+  for (int j = 0; j < 7; ++j) a[j] = r[j];
+}
+
+// One level, or (word set) all levels from the root down, a grid barrier between
+// them; the list entries of a group's first twig of the next level are read before it.
+__global__ void __launch_bounds__(kDownThreads) k_adj_down(int level, int last, DownArgs D,
+                                                           unsigned* word, uint32_t* status) {
+  __shared__ int s_cnt[kMaxLevel + 1], s_base[kMaxLevel + 1];
+  if (threadIdx.x <= kMaxLevel) {
+    int base = 0;
+    for (int l = 0; l < (int)threadIdx.x; ++l) base += D.lvl[l];
+    s_base[threadIdx.x] = base;
+    s_cnt[threadIdx.x] = D.lvl[threadIdx.x];
+  }
+  __syncthreads();
+  const int step = gridDim.x * (kDownThreads / 8);
+  const int first = blockIdx.x * (kDownThreads / 8) + (threadIdx.x >> 3);
+  unsigned barriers = 0;
+  DownHead h = down_head(D, s_base[level] + first, first < s_cnt[level]);
+  for (; level <= last; ++level) {
+    const int cnt = s_cnt[level], base = s_base[level];
+    for (int i0 = blockIdx.x * (kDownThreads / 8), i = first; i0 < cnt; i0 += step, i += step) {
+      if (i != first) h = down_head(D, base + i, i < cnt);
+      adj_down_twig(D, h);
+      __syncwarp();
+    }
+    if (level < last) {
+      h = down_head(D, s_base[level + 1] + first, first < s_cnt[level + 1]);
+      if (gridDim.x > 1) {
+        if (!grid_barrier(word, ++barriers * gridDim.x, status)) return;
       } else {
-        for (int j = 0; j < 3; ++j) a[10 + j] += cocbar[j] / (double)nc;
+        __syncthreads();
       }
     }
   }
@@ -604,6 +660,46 @@ void launch_adj_law(int law, bool per_target, int tpl, bool with_e, int blocks, 
   if (law == 2) launch_adj<2>(per_target, tpl, with_e, blocks, s, A);
   else if (law == 4) launch_adj<4>(per_target, tpl, with_e, blocks, s, A);
   else launch_adj<3>(per_target, tpl, with_e, blocks, s, A);
+}
+
+// Pass 2: in one launch, or by level.  Whole adjoint call with 500 targets, ms, by level /
+// one launch: 262,144 sources 0.331 / 0.315, 1,000,000 (widest level 160,000) 0.646 /
+// 0.633, 4,000,000 (640,000) 2.47 / 3.24: the resident blocks are then too few for the
+// widest levels' loads.
+constexpr int kDownFusedWidest = 170000;
+bool downward_pass(Ctx* c, cudaStream_t s) {
+  const DownArgs D{c->lvlcnt.p, c->tinfo.p, c->tcounts.p, c->tcounts.p + c->ntwig, c->drec.p,
+                   c->dmom.p, c->adj.p};
+  int64_t widest = 0;
+  for (int L = 0; L < c->max_level; ++L) widest = std::max<int64_t>(widest, c->lvl_host[L]);
+  constexpr int kTwigs = kDownThreads / 8;
+  if (widest <= kDownFusedWidest) {
+    if (!cuda_ok(c, cudaMemsetAsync(c->barrier_word(2), 0, sizeof(unsigned), s), "adjoint")) return false;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)std::min<int64_t>((widest + kTwigs - 1) / kTwigs,
+                                                   widest > 16384 ? 592 : 296));
+    cfg.blockDim = dim3(kDownThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_adj_down, 0, c->max_level - 1, D, c->barrier_word(2),
+                           c->d_status + 1) == cudaSuccess) {
+      COUNT_LAUNCH();
+      return true;
+    }
+    cudaGetLastError();  // level by level instead
+  }
+  for (int L = 0; L < c->max_level; ++L) {
+    const int64_t cnt = c->lvl_host[L];
+    if (cnt <= 0) continue;
+    COUNT_LAUNCH();
+    const unsigned gl = (unsigned)std::min<int64_t>((cnt + kTwigs - 1) / kTwigs, 148 * 16);
+    k_adj_down<<<gl, kDownThreads, 0, s>>>(L, L, D, nullptr, c->d_status);
+  }
+  return true;
 }
 
 }  // namespace
@@ -715,15 +811,7 @@ int adjoint_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const
     launch_adj_law(c->prm.force_law, per_target, tpl, h_flag != 0, blocks, s, A);
   }
   const unsigned g = (unsigned)((M + 255) / 256 > 148 * 16 ? 148 * 16 : (M + 255) / 256);
-  for (int L = 0; L < c->max_level; ++L) {
-    const int64_t cnt = c->lvl_host[L];
-    if (cnt <= 0) continue;
-    const unsigned gl = (unsigned)std::min<int64_t>((cnt + 255) / 256, 148 * 16);
-    COUNT_LAUNCH();
-    k_adj_down_level<<<gl, 256, 0, s>>>(L, c->lvlcnt.p, c->twiglist.p, c->tinfo.p,
-                                        c->tcounts.p, c->tcounts.p + c->ntwig, c->drec.p,
-                                        c->dmom.p, c->adj.p);
-  }
+  if (!downward_pass(c, s)) return PEPCG_ERR_CUDA;
   COUNT_LAUNCH();
   k_adj_out<<<g, 256, 0, s>>>(c->n, c->leafnode.p, c->lvlpos.p, c->perm.p, c->q.p, c->adj.p, dq,
                               dx, dy, dz);

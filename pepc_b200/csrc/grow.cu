@@ -1737,7 +1737,7 @@ static void upward_pass(Ctx* c, const UpArgs& U, cudaStream_t s) {
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_upward_all, c->max_level - 1, U, c->barrier_word(1), c->d_status) ==
+    if (cudaLaunchKernelEx(&cfg, k_upward_all, c->max_level - 1, U, c->barrier_word(1), c->d_status + 1) ==
         cudaSuccess) {
       COUNT_LAUNCH();
       return;
@@ -1782,7 +1782,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
       !ensure(c, c->packed, n, "packed"))
     return PEPCG_ERR_OOM;
 
-  if (!cuda_ok(c, cudaMemsetAsync(c->d_status, 0, sizeof(uint32_t), s), "memset status") ||
+  if (!cuda_ok(c, cudaMemsetAsync(c->d_status, 0, 2 * sizeof(uint32_t), s), "memset status") ||
       !cuda_ok(c, cudaMemsetAsync(c->d_small, 0, 32 * sizeof(unsigned long long), s), "memset") ||
       !cuda_ok(c, cudaMemsetAsync(c->lvlcnt.p, 0, 64 * sizeof(int32_t), s), "memset lvl"))
     return PEPCG_ERR_CUDA;

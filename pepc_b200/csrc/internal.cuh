@@ -196,11 +196,13 @@ struct Ctx {
   DBuf<int64_t> tkeys;
   // small device state: box (9), boxlength2 (21), status word, dup count ...
   double* d_box = nullptr;    // [0..8] box, [9..29] boxlength2
+  // status words: [0] of the running call, [1] of the tree's later kernels (upward pass,
+  // adjoint), which nothing waits for: read with the next walk's status
   uint32_t* d_status = nullptr;
   unsigned long long* d_small = nullptr;  // [0] dup count, [1] nnodes, [2] tile count, ...
                                           // [8], [9] walk bucket queues (one per walk
                                           // stream), [10] adjoint item queue,
-                                          // [16], [17] grid barriers
+                                          // [16] .. [17] grid barriers (32-bit words)
   double box[9];
   double boxlength2[kMaxLevel + 1];
   int max_level = 0;

@@ -1126,7 +1126,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   cudaEventRecord(c->ev[7], s);
   if (plan && plan->before_sync && !plan->before_sync()) return PEPCG_ERR_CUDA;
   unsigned long long ctr[4];
-  uint32_t st = 0;
+  uint32_t st[2] = {0, 0};  // this walk's, and the tree's (see Ctx::d_status)
   int32_t nover = 0;
   if (lists) {
     if (!cuda_ok(c, cudaMemcpyAsync(&nover, c->over.p, sizeof(nover), cudaMemcpyDeviceToHost, s), "walk lists") ||
@@ -1145,7 +1145,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   }
   if (!cuda_ok(c, cudaMemcpyAsync(ctr, c->counters.p, 4 * sizeof(unsigned long long),
                                   cudaMemcpyDeviceToHost, s), "counters") ||
-      !cuda_ok(c, cudaMemcpyAsync(&st, c->d_status, 4, cudaMemcpyDeviceToHost, s), "status") ||
+      !cuda_ok(c, cudaMemcpyAsync(st, c->d_status, 8, cudaMemcpyDeviceToHost, s), "status") ||
       !cuda_ok(c, cudaStreamSynchronize(s), "walk"))
     return PEPCG_ERR_CUDA;
   c->st.leaf_interactions = (int64_t)ctr[0];
@@ -1155,7 +1155,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   float ms = 0;
   if (cudaEventElapsedTime(&ms, c->ev[5], c->ev[6]) == cudaSuccess) c->st.t_walk_ms = ms;
   if (cudaEventElapsedTime(&ms, c->ev[6], c->ev[7]) == cudaSuccess) c->st.t_lattice_ms = ms;
-  if (st) return status_to_code(c, st);
+  if (st[0] | st[1]) return status_to_code(c, st[0] | st[1]);
   return PEPCG_OK;
 }
 
