@@ -104,54 +104,66 @@ __device__ __forceinline__ void twig32(float4 m0, float4 m1, float4 m2, float dx
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 
-// twig32 for two targets against the same node in packed FP32 (sm_100
-// FFMA2 / FMUL2 / FADD2): each operation evaluates both targets' terms, and
-// the node's moments enter as (m, m) pairs.  Per target the arithmetic is
-// twig32's, operation for operation.
+// -a by the sign bits (integer operations: the FMA pipe is the busy one)
+__device__ __forceinline__ float2 neg2(float2 a) {
+  return make_float2(__uint_as_float(__float_as_uint(a.x) ^ 0x80000000u),
+                     __uint_as_float(__float_as_uint(a.y) ^ 0x80000000u));
+}
+
+// twig32's interaction for two targets against the same node in packed FP32
+// (sm_100 FFMA2 / FMUL2 / FADD2): each operation evaluates both targets' terms, and
+// the node's moments enter as (m, m) pairs.  With s1 = A - B/r^2 and s2 = s1 - B/r^2,
+//   phi = (q - s1/r^2) / r,   5B/r^2 - 3A = -(s1 + 2 s2),
+// so E's coefficient of d follows from phi's inner term g = q - s1/r^2 as
+// g - 2 s2/r^2: one operation less than twig32's form.
+struct Twig2 {
+  float2 ri, rd3, g, ex, ey, ez;  // phi = ri g, E = rd3 e
+};
+__device__ __forceinline__ Twig2 twig32x2_parts(float4 m0, float4 m1, float4 m2, float2 dx,
+                                                float2 dy, float2 dz, float2 eps2) {
+  const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, eps2)));
+  const float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+  const float2 ri2 = __fmul2_rn(ri, ri);
+  const float2 n2 = neg2(ri2);
+  const float2 m2r = __fmul2_rn(f2(-2.0f), ri2);
+  const float2 A = __ffma2_rn(dx, f2(m0.x), __ffma2_rn(dy, f2(m0.y), __ffma2_rn(dz, f2(m0.z), f2(m2.y))));
+  const float2 vx = __ffma2_rn(f2(m0.w), dx, __ffma2_rn(f2(m1.z), dy, __fmul2_rn(f2(m2.x), dz)));
+  const float2 vy = __ffma2_rn(f2(m1.z), dx, __ffma2_rn(f2(m1.x), dy, __fmul2_rn(f2(m1.w), dz)));
+  const float2 vz = __ffma2_rn(f2(m2.x), dx, __ffma2_rn(f2(m1.w), dy, __fmul2_rn(f2(m1.y), dz)));
+  const float2 B = __ffma2_rn(dx, vx, __ffma2_rn(dy, vy, __fmul2_rn(dz, vz)));
+  const float2 s1 = __ffma2_rn(n2, B, A);
+  const float2 g = __ffma2_rn(n2, s1, f2(m2.z));
+  const float2 t4 = __ffma2_rn(m2r, __ffma2_rn(n2, B, s1), g);
+  Twig2 t;
+  t.ri = ri;
+  t.rd3 = __fmul2_rn(ri, ri2);
+  t.g = g;
+  t.ex = __ffma2_rn(t4, dx, __ffma2_rn(m2r, vx, f2(m0.x)));
+  t.ey = __ffma2_rn(t4, dy, __ffma2_rn(m2r, vy, f2(m0.y)));
+  t.ez = __ffma2_rn(t4, dz, __ffma2_rn(m2r, vz, f2(m0.z)));
+  return t;
+}
+
 __device__ __forceinline__ void twig32x2(float4 m0, float4 m1, float4 m2, float2 dx, float2 dy,
                                          float2 dz, float2 eps2, float2& ax, float2& ay,
                                          float2& az, float2& ap) {
-  const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, eps2)));
-  const float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
-  const float2 ri2 = __fmul2_rn(ri, ri);
-  const float2 rd3 = __fmul2_rn(ri, ri2);
-  const float2 q = f2(m2.z);
-  const float2 A = __ffma2_rn(dx, f2(m0.x), __ffma2_rn(dy, f2(m0.y), __ffma2_rn(dz, f2(m0.z), f2(m2.y))));
-  const float2 vx = __ffma2_rn(f2(m0.w), dx, __ffma2_rn(f2(m1.z), dy, __fmul2_rn(f2(m2.x), dz)));
-  const float2 vy = __ffma2_rn(f2(m1.z), dx, __ffma2_rn(f2(m1.x), dy, __fmul2_rn(f2(m1.w), dz)));
-  const float2 vz = __ffma2_rn(f2(m2.x), dx, __ffma2_rn(f2(m1.w), dy, __fmul2_rn(f2(m1.y), dz)));
-  const float2 B = __ffma2_rn(dx, vx, __ffma2_rn(dy, vy, __fmul2_rn(dz, vz)));
-  const float2 t1 = __ffma2_rn(ri2, B, make_float2(-A.x, -A.y));
-  ap = __ffma2_rn(ri, __ffma2_rn(ri2, t1, q), ap);
-  const float2 t4 = __ffma2_rn(ri2, __ffma2_rn(f2(5.0f), t1, __fadd2_rn(A, A)), q);
-  const float2 m2r = __fmul2_rn(f2(-2.0f), ri2);
-  ax = __ffma2_rn(rd3, __ffma2_rn(t4, dx, __ffma2_rn(m2r, vx, f2(m0.x))), ax);
-  ay = __ffma2_rn(rd3, __ffma2_rn(t4, dy, __ffma2_rn(m2r, vy, f2(m0.y))), ay);
-  az = __ffma2_rn(rd3, __ffma2_rn(t4, dz, __ffma2_rn(m2r, vz, f2(m0.z))), az);
+  const Twig2 t = twig32x2_parts(m0, m1, m2, dx, dy, dz, eps2);
+  ap = __ffma2_rn(t.ri, t.g, ap);
+  ax = __ffma2_rn(t.rd3, t.ex, ax);
+  ay = __ffma2_rn(t.rd3, t.ey, ay);
+  az = __ffma2_rn(t.rd3, t.ez, az);
 }
 
-// twig32x2's terms of one interaction, returned instead of accumulated (the
-// strict form adds them with compensation)
+// the terms of one interaction, returned instead of accumulated (the strict form
+// adds them with compensation)
 __device__ __forceinline__ void twig32x2_terms(float4 m0, float4 m1, float4 m2, float2 dx,
                                                float2 dy, float2 dz, float2 eps2, float2& ax,
                                                float2& ay, float2& az, float2& ap) {
-  const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, eps2)));
-  const float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
-  const float2 ri2 = __fmul2_rn(ri, ri);
-  const float2 rd3 = __fmul2_rn(ri, ri2);
-  const float2 q = f2(m2.z);
-  const float2 A = __ffma2_rn(dx, f2(m0.x), __ffma2_rn(dy, f2(m0.y), __ffma2_rn(dz, f2(m0.z), f2(m2.y))));
-  const float2 vx = __ffma2_rn(f2(m0.w), dx, __ffma2_rn(f2(m1.z), dy, __fmul2_rn(f2(m2.x), dz)));
-  const float2 vy = __ffma2_rn(f2(m1.z), dx, __ffma2_rn(f2(m1.x), dy, __fmul2_rn(f2(m1.w), dz)));
-  const float2 vz = __ffma2_rn(f2(m2.x), dx, __ffma2_rn(f2(m1.w), dy, __fmul2_rn(f2(m1.y), dz)));
-  const float2 B = __ffma2_rn(dx, vx, __ffma2_rn(dy, vy, __fmul2_rn(dz, vz)));
-  const float2 t1 = __ffma2_rn(ri2, B, make_float2(-A.x, -A.y));
-  ap = __fmul2_rn(ri, __ffma2_rn(ri2, t1, q));
-  const float2 t4 = __ffma2_rn(ri2, __ffma2_rn(f2(5.0f), t1, __fadd2_rn(A, A)), q);
-  const float2 m2r = __fmul2_rn(f2(-2.0f), ri2);
-  ax = __fmul2_rn(rd3, __ffma2_rn(t4, dx, __ffma2_rn(m2r, vx, f2(m0.x))));
-  ay = __fmul2_rn(rd3, __ffma2_rn(t4, dy, __ffma2_rn(m2r, vy, f2(m0.y))));
-  az = __fmul2_rn(rd3, __ffma2_rn(t4, dz, __ffma2_rn(m2r, vz, f2(m0.z))));
+  const Twig2 t = twig32x2_parts(m0, m1, m2, dx, dy, dz, eps2);
+  ap = __fmul2_rn(t.ri, t.g);
+  ax = __fmul2_rn(t.rd3, t.ex);
+  ay = __fmul2_rn(t.rd3, t.ey);
+  az = __fmul2_rn(t.rd3, t.ez);
 }
 
 // Kahan (compensated) summation, both lanes of a pair: s += v with the
@@ -190,6 +202,19 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int& total) {
   }
   total = __shfl_sync(0xffffffffu, x, 31);
   return x - v;
+}
+
+// exclusive prefix of v in 0 .. 8 over the warp, from one ballot per bit
+__device__ __forceinline__ int warp_excl_scan8(int v, unsigned lt, int& total) {
+  int off = 0;
+  total = 0;
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    const unsigned m = __ballot_sync(0xffffffffu, (v >> b) & 1);
+    off += __popc(m & lt) << b;
+    total += __popc(m) << b;
+  }
+  return off;
 }
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -351,10 +376,11 @@ __device__ __forceinline__ unsigned leaf_batch64(const StagedLeaf* ring, int hea
       const bool za = d2.x == 0.f, zb = v1 && d2.y == 0.f;
       pend |= (za || zb) ? (1u << k) : 0u;
       const float2 wq = make_float2(za ? 0.f : c.w, zb ? 0.f : c.w);
-      // the pair's leaf32 in packed FP32; a zero r2 (eps2 = 0) gives no
-      // contribution instead of inf
-      const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, E2)));
-      const float2 ri = make_float2(r2.x > 0.f ? rsqrt_ftz(r2.x) : 0.f, r2.y > 0.f ? rsqrt_ftz(r2.y) : 0.f);
+      // the pair's leaf32 in packed FP32.  A zero r2 (eps2 = 0) comes with charge 0
+      // and gives no contribution: the bound keeps its rsqrt finite, and lies below
+      // any square of an offset that is not zero in FP32 at a scale >= 1e-18
+      const float2 r2 = __fadd2_rn(d2, E2);
+      const float2 ri = make_float2(rsqrt_ftz(fmaxf(r2.x, 1e-37f)), rsqrt_ftz(fmaxf(r2.y, 1e-37f)));
       const float2 qr = __fmul2_rn(wq, ri);
       const float2 qr3 = __fmul2_rn(__fmul2_rn(qr, ri), ri);
       PP = __fadd2_rn(PP, qr);

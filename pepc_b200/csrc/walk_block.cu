@@ -212,10 +212,12 @@ __device__ __forceinline__ bool block_traverse(const BlockTree& B, const BucketL
         const float uy = __shfl_sync(0xffffffffu, d.cy, j);
         const float uz = __shfl_sync(0xffffffffu, d.cz, j);
         const float ub = __shfl_sync(0xffffffffu, bl, j);
-        float dx = K.T.rxa - ux, dy = K.T.rya - uy, dz = K.T.rza - uz;
-        fa = K.v0 && !(theta2 * fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > ub);
-        dx = K.T.rxb - ux; dy = K.T.ryb - uy; dz = K.T.rzb - uz;
-        fb = K.v1 && !(theta2 * fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > ub);
+        const float2 dx = __fadd2_rn(make_float2(K.T.rxa, K.T.rxb), f2(-ux)),
+                     dy = __fadd2_rn(make_float2(K.T.rya, K.T.ryb), f2(-uy)),
+                     dz = __fadd2_rn(make_float2(K.T.rza, K.T.rzb), f2(-uz));
+        const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+        fa = K.v0 && !(theta2 * d2.x > ub);
+        fb = K.v1 && !(theta2 * d2.y > ub);
       }
       const unsigned f0 = __ballot_sync(0xffffffffu, fa);
       const unsigned f1 = __ballot_sync(0xffffffffu, fb);
@@ -233,7 +235,7 @@ __device__ __forceinline__ bool block_traverse(const BlockTree& B, const BucketL
     const unsigned ab = __ballot_sync(0xffffffffu, accept && mine);
     const int npush = open ? min(8, d.lk.y >> 16) : 0;
     int wtotal;
-    int off = warp_excl_scan(npush, lane, wtotal);
+    int off = warp_excl_scan8(npush, lt, wtotal);
     if (lane == 0) s_cnt[w] = make_uint2((unsigned)__popc(lb) | ((unsigned)__popc(ab) << 16), (unsigned)wtotal);
     __syncthreads();  // the counts are in; every thread has read its stack entry
     const uint2 c = lane < W ? s_cnt[lane] : make_uint2(0u, 0u);
@@ -588,7 +590,8 @@ bool launch_block(Ctx* c, K kern, int threads, size_t smem, int blocks, int npar
 
 }  // namespace
 
-// Measured (walk ms, Plummer, theta 0.4, one warp per bucket -> the choice here):
+// Measured when the choice was made (walk ms, Plummer, theta 0.4, one warp per bucket ->
+// the choice here; both are some per cent faster since):
 // 16 buckets 0.182 -> 0.044, 64: 0.48 -> 0.064, 141: 0.74 -> 0.114, 257: 1.04 -> 0.21,
 // 516: 1.29 -> 0.36, 938: 1.44 -> 0.59, 1,563: 1.60 -> 0.92, 3,126: 1.83 -> 1.78, and past
 // that one warp per bucket is faster (6,250: 3.48 against 3.62).  Eight warps at two blocks
