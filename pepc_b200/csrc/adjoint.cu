@@ -668,7 +668,7 @@ void launch_adj_law(int law, bool per_target, int tpl, bool with_e, int blocks, 
 // widest levels' loads.
 constexpr int kDownFusedWidest = 170000;
 bool downward_pass(Ctx* c, cudaStream_t s) {
-  const DownArgs D{c->lvlcnt.p, c->tinfo.p, c->tcounts.p, c->tcounts.p + c->ntwig, c->drec.p,
+  const DownArgs D{c->lvlcnt, c->tinfo.p, c->tcounts.p, c->tcounts.p + c->ntwig, c->drec.p,
                    c->dmom.p, c->adj.p};
   int64_t widest = 0;
   for (int L = 0; L < c->max_level; ++L) widest = std::max<int64_t>(widest, c->lvl_host[L]);

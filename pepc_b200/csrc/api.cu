@@ -344,8 +344,8 @@ int pepcg_create(void** out, const pepcg_params* p) {
   c->own_stream = true;
   for (int i = 0; i < Ctx::kEvents; ++i) cudaEventCreate(&c->ev[i]);
   bool ok = cuda_ok(nullptr, cudaMalloc((void**)&c->d_box, 64 * sizeof(double)), "box") &&
-            cuda_ok(nullptr, cudaMalloc((void**)&c->d_status, 16), "status") &&
-            cuda_ok(nullptr, cudaMalloc((void**)&c->d_small, 32 * sizeof(unsigned long long)), "small") &&
+            cuda_ok(nullptr, cudaMalloc((void**)&c->d_small, Ctx::kSmall * sizeof(unsigned long long)),
+                    "small") &&
             cuda_ok(nullptr, cudaMalloc((void**)&c->d_vbox, 3 * 125 * sizeof(double)), "vbox") &&
             cuda_ok(nullptr, cudaMalloc((void**)&c->d_part, 6 * 512 * sizeof(double)), "part") &&
             cuda_ok(nullptr, cudaHostAlloc((void**)&c->h_sum, sizeof(Ctx::GrowSummary),
@@ -357,6 +357,8 @@ int pepcg_create(void** out, const pepcg_params* p) {
     pepcg_destroy(c);
     return PEPCG_ERR_CUDA;
   }
+  c->d_status = reinterpret_cast<uint32_t*>(c->d_small + 32);
+  c->lvlcnt = reinterpret_cast<int32_t*>(c->d_small + 34);
   prepare_boxes(c);
   cudaMemcpy(c->d_vbox, c->vbox, 3 * c->nboxes * sizeof(double), cudaMemcpyHostToDevice);
   if (!ensure(c, c->counters, 8, "counters")) {
@@ -391,13 +393,13 @@ int pepcg_destroy(void* ctx) {
   release(c->scan_tmp);
   release(c->nc4); release(c->meta); release(c->fwd); release(c->fwdf); release(c->tflag); release(c->tpack); release(c->mom);
   release(c->mom32);
-  release(c->parent); release(c->nchild); release(c->twiglist); release(c->lvlcnt); release(c->lvlblk);
+  release(c->parent); release(c->nchild); release(c->twiglist); release(c->lvlblk);
   release(c->drec); release(c->lvlpos); release(c->dmom);
   release(c->tinfo); release(c->tcounts); release(c->macb); release(c->first_part);
   release(c->nleaves); release(c->child8); release(c->wstack); release(c->over); release(c->leafnode);
   release(c->adj); release(c->fpo2rpo); release(c->rpo2fpo); release(c->nkey);
   release(c->tiles); release(c->counters); release(c->tgt); release(c->tkeys);
-  for (void* p : {(void*)c->d_box, (void*)c->d_status, (void*)c->d_small, (void*)c->d_vbox,
+  for (void* p : {(void*)c->d_box, (void*)c->d_small, (void*)c->d_vbox,
                   (void*)c->d_part, (void*)c->d_mlattice, (void*)c->d_lattab, (void*)c->d_latcoef,
                   (void*)c->d_latpart, (void*)c->d_ofict, (void*)c->d_site, (void*)c->d_site_q,
                   (void*)c->d_site_n, (void*)c->d_fmm_aux, (void*)c->d_factorial})

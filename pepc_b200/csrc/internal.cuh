@@ -171,7 +171,7 @@ struct Ctx {
   DBuf<float> mom32;  // 16 floats per node (64 B): the FP32 moments, padded
   DBuf<int32_t> parent, nchild, first_part, nleaves;
   DBuf<int32_t> twiglist;  // twig RPO indices grouped by level (upward and adjoint passes)
-  DBuf<int32_t> lvlcnt;    // [0, 32) twigs per level
+  int32_t* lvlcnt = nullptr;  // twigs per level (in d_small's block)
   DBuf<int32_t> lvlblk;    // twigs, then nodes, per (level, block of 256 nodes), scanned
   // level-ordered copy of the node records for the upward pass: centre /
   // charge and (abs_charge, bmax); the twigs' moments by twig-list position
@@ -202,7 +202,10 @@ struct Ctx {
   unsigned long long* d_small = nullptr;  // [0] dup count, [1] nnodes, [2] tile count, ...
                                           // [8], [9] walk bucket queues (one per walk
                                           // stream), [10] adjoint item queue,
-                                          // [16] .. [17] grid barriers (32-bit words)
+                                          // [16] .. [19] grid barriers and block
+                                          // counters (32-bit words); then d_status
+                                          // and lvlcnt, so that one memset clears all
+  static constexpr int kSmall = 34 + 16;
   double box[9];
   double boxlength2[kMaxLevel + 1];
   int max_level = 0;
