@@ -626,11 +626,14 @@ __global__ void k_reset_adj(unsigned int* q, unsigned long long* items) {
   *items = 0;
 }
 
+// *flag (mapped host memory, zero before the launch) = 1 if any value is not zero
 __global__ void k_any_nonzero(int64_t n, const double* a, const double* b, const double* c,
-                              unsigned int* flag) {
+                              uint32_t* flag) {
+  bool any = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
-    if (a[i] != 0.0 || b[i] != 0.0 || c[i] != 0.0) atomicOr(flag, 1u);
+    any |= a[i] != 0.0 || b[i] != 0.0 || c[i] != 0.0;
+  if (__syncthreads_or(any) && threadIdx.x == 0) *flag = 1u;
 }
 
 // the group walk's buckets of bs key-consecutive targets as (first, count)
@@ -724,11 +727,9 @@ int adjoint_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const
   if (!cuda_ok(c, cudaMemsetAsync(c->adj.p, 0, sizeof(double) * kNA * M, s), "adjoint"))
     return PEPCG_ERR_CUDA;
   // is dL/dE zero everywhere?  (then the Hessian terms are skipped)
-  unsigned int* d_flag = reinterpret_cast<unsigned int*>(c->d_small + 6);
-  unsigned int h_flag = 1;
-  cudaMemsetAsync(d_flag, 0, 4, s);
+  c->h_sum->with_e = 0;  // every earlier call that wrote it has been waited for
   COUNT_LAUNCH();
-  k_any_nonzero<<<148, 256, 0, s>>>(nt, gex, gey, gez, d_flag);
+  k_any_nonzero<<<148, 256, 0, s>>>(nt, gex, gey, gez, &c->d_sum->with_e);
   AdjArgs A;
   A.nt = nt;
   A.tx = tx; A.ty = ty; A.tz = tz;
@@ -796,9 +797,8 @@ int adjoint_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const
     A.tiles = d_tiles;
     A.ntiles = ntiles;
   }
-  if (!cuda_ok(c, cudaMemcpyAsync(&h_flag, d_flag, 4, cudaMemcpyDeviceToHost, s), "flag") ||
-      !cuda_ok(c, cudaStreamSynchronize(s), "flag"))
-    return PEPCG_ERR_CUDA;
+  if (!cuda_ok(c, cudaStreamSynchronize(s), "flag")) return PEPCG_ERR_CUDA;
+  const uint32_t h_flag = *const_cast<volatile uint32_t*>(&c->h_sum->with_e);
   COUNT_LAUNCH();
   k_reset_adj<<<1, 1, 0, s>>>(A.queue, A.item_queue);
   const int blocks = 148 * 8;

@@ -222,6 +222,10 @@ struct Ctx {
     int32_t max_level;
     int32_t lvl[kMaxLevel + 1];
     uint32_t not_neutral;           // the lattice step found a net charge
+    unsigned long long ctr[3];      // of the last walk: leaf, twig, MAC counts,
+    uint32_t walk_status;           // status words, buckets left to the warp walks
+    int32_t nover;
+    uint32_t with_e;                // the adjoint's dL/dE is not zero everywhere
   };
   GrowSummary* h_sum = nullptr;  // host address
   GrowSummary* d_sum = nullptr;  // its device address

@@ -68,6 +68,7 @@ struct WalkArgs {
   const int32_t* rpo2fpo;
   const int32_t* fpo2rpo;
   uint2* lstack;       // kListStack entries per resident block
+  int lper;            // per target: targets per bucket (8, 16 or 32)
   // buckets (packs) whose lists did not fit: [0] their number, then their indices.
   // Written by k_walk_list64; k_walk_target64 / k_walk_tilepack64 walk them (kOnly)
   int32_t* over;
@@ -116,9 +117,10 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_target64(WalkArgs A) {
       if ((int)b >= A.over[0]) break;
       b = (unsigned)A.over[1 + b];
     }
-    if ((int64_t)b * 32 >= A.nt) break;
-    const int64_t t = (int64_t)b * 32 + lane;
-    const bool valid = t < A.nt;
+    const int per = kOnly ? A.lper : 32;
+    if ((int64_t)b * per >= A.nt) break;
+    const int64_t t = (int64_t)b * per + lane;
+    const bool valid = t < A.nt && (!kOnly || lane < per);
     double px = 0, py = 0, pz = 0, e0 = 0, e1 = 0, e2 = 0, ph = 0, w = 0;
     KelbgArgs kel{0.0, A.kinv, A.sqrtpi};
     if (valid) {
@@ -476,7 +478,7 @@ __global__ void __launch_bounds__(kListThreads, 2) k_walk_list64(WalkArgs A) {
   const unsigned lt = (1u << lane) - 1u;
   for (int i = tid; i <= kMaxLevel; i += kListThreads) S.bl2[i] = A.bl2[i];
   uint2* stack = A.lstack + (int64_t)blockIdx.x * kListStack;
-  const int64_t nbk = kTile ? (int64_t)*A.npacks : (A.nt + 31) / 32;
+  const int64_t nbk = kTile ? (int64_t)*A.npacks : (A.nt + A.lper - 1) / A.lper;
   const double vx = A.vbox[0], vy = A.vbox[1], vz = A.vbox[2];
   unsigned long long c_leaf = 0, c_twig = 0, c_mac = 0;
   for (;;) {
@@ -494,8 +496,8 @@ __global__ void __launch_bounds__(kListThreads, 2) k_walk_list64(WalkArgs A) {
       valid = pack_lane(A.pstart, A.tflag, b, lane, tl0, len);
       tmask = valid ? (((len >= 32) ? 0xffffffffu : ((1u << len) - 1u)) << tl0) : 0u;
     } else {
-      t0 = b * 32;
-      valid = t0 + lane < A.nt;
+      t0 = b * A.lper;
+      valid = lane < A.lper && t0 + lane < A.nt;
     }
     const unsigned all = __ballot_sync(0xffffffffu, valid);
     if (all == 0u) {
@@ -904,6 +906,24 @@ static bool use_list_walk(const Ctx* c, int64_t nt, bool chunked, bool packed) {
   return c->nnodes <= kListCap || (p.mac_select == 0 && p.theta2 >= 0.12);
 }
 
+// Targets per bucket of the per-target walk: a bucket's search and its batches are a
+// serial chain, so few targets take small buckets, as long as two blocks per SM hold
+// them all.  Walk ms with 32 / 16 / 8: 1,000 targets 0.078 / 0.065 / 0.057, 4,099: 0.116 /
+// 0.090 / 0.120, 8,000: 0.133 / 0.166 / 0.227.
+static int list_bucket(int64_t nt) {
+  return nt <= 8 * kListBlocks ? 8 : nt <= 16 * kListBlocks ? 16 : 32;
+}
+
+// What the host needs of a finished walk, into mapped host memory (two or three
+// device-to-host copies to pageable memory and their staging took 10 us more).
+static __global__ void k_walk_summary(const unsigned long long* __restrict__ ctr,
+                                      const uint32_t* __restrict__ status,
+                                      const int32_t* __restrict__ over, Ctx::GrowSummary* out) {
+  if (threadIdx.x < 3) out->ctr[threadIdx.x] = ctr[threadIdx.x];
+  if (threadIdx.x == 3) out->walk_status = status[0] | status[1];  // see Ctx::d_status
+  if (threadIdx.x == 4) out->nover = over ? *over : 0;
+}
+
 int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const double* tz,
                     const int64_t* tkeys, bool self, double* ex, double* ey, double* ez,
                     double* pot, double* work, const double* tq, const ChunkPlan* plan,
@@ -1040,7 +1060,9 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   const int blocks = 148 * 8;
   const bool lists = use_list_walk(c, nt, plan != nullptr, packed);
   if (lists) {
-    const int64_t nbk = packed ? (nt + kPackChunk - 1) / kPackChunk * kPackSlots : (nt + 31) / 32;
+    A.lper = list_bucket(nt);
+    const int64_t nbk = packed ? (nt + kPackChunk - 1) / kPackChunk * kPackSlots
+                               : (nt + A.lper - 1) / A.lper;
     if (!ensure(c, c->wstack, (size_t)2 * kListStack * kListBlocks, "walk stacks") ||
         !ensure(c, c->over, nbk + 1, "walk lists"))
       return PEPCG_ERR_OOM;
@@ -1125,29 +1147,25 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   }
   cudaEventRecord(c->ev[7], s);
   if (plan && plan->before_sync && !plan->before_sync()) return PEPCG_ERR_CUDA;
-  unsigned long long ctr[4];
-  uint32_t st[2] = {0, 0};  // this walk's, and the tree's (see Ctx::d_status)
-  int32_t nover = 0;
-  if (lists) {
-    if (!cuda_ok(c, cudaMemcpyAsync(&nover, c->over.p, sizeof(nover), cudaMemcpyDeviceToHost, s), "walk lists") ||
-        !cuda_ok(c, cudaStreamSynchronize(s), "walk lists"))
-      return PEPCG_ERR_CUDA;
-    if (nover > 0) {  // lists that did not fit: these buckets by the warp walks
-      COUNT_LAUNCH();
-      k_reset_counter<<<1, 1, 0, s>>>(A.queue);
-      COUNT_LAUNCH();
-      if (packed) k_walk_tilepack64<3, false, true><<<blocks, kWalkThreads, 0, s>>>(A);
-      else k_walk_target64<3, false, true><<<blocks, kWalkThreads, 0, s>>>(A);
-      cudaEventRecord(c->ev[6], s);
-      cudaEventRecord(c->ev[7], s);
-      if (!cuda_ok(c, cudaGetLastError(), "walk launch")) return PEPCG_ERR_CUDA;
-    }
+  auto summary = [&]() {
+    COUNT_LAUNCH();
+    k_walk_summary<<<1, 32, 0, s>>>(c->counters.p, c->d_status, lists ? c->over.p : nullptr, c->d_sum);
+    return cuda_ok(c, cudaGetLastError(), "walk summary") &&
+           cuda_ok(c, cudaStreamSynchronize(s), "walk");
+  };
+  if (!summary()) return PEPCG_ERR_CUDA;
+  if (lists && c->h_sum->nover > 0) {  // lists that did not fit: these buckets by the warp walks
+    COUNT_LAUNCH();
+    k_reset_counter<<<1, 1, 0, s>>>(A.queue);
+    COUNT_LAUNCH();
+    if (packed) k_walk_tilepack64<3, false, true><<<blocks, kWalkThreads, 0, s>>>(A);
+    else k_walk_target64<3, false, true><<<blocks, kWalkThreads, 0, s>>>(A);
+    cudaEventRecord(c->ev[6], s);
+    cudaEventRecord(c->ev[7], s);
+    if (!summary()) return PEPCG_ERR_CUDA;
   }
-  if (!cuda_ok(c, cudaMemcpyAsync(ctr, c->counters.p, 4 * sizeof(unsigned long long),
-                                  cudaMemcpyDeviceToHost, s), "counters") ||
-      !cuda_ok(c, cudaMemcpyAsync(st, c->d_status, 8, cudaMemcpyDeviceToHost, s), "status") ||
-      !cuda_ok(c, cudaStreamSynchronize(s), "walk"))
-    return PEPCG_ERR_CUDA;
+  const unsigned long long* ctr = c->h_sum->ctr;
+  const uint32_t st = c->h_sum->walk_status;
   c->st.leaf_interactions = (int64_t)ctr[0];
   c->st.twig_interactions = (int64_t)ctr[1];
   c->st.interactions = (int64_t)(ctr[0] + ctr[1]);
@@ -1155,7 +1173,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   float ms = 0;
   if (cudaEventElapsedTime(&ms, c->ev[5], c->ev[6]) == cudaSuccess) c->st.t_walk_ms = ms;
   if (cudaEventElapsedTime(&ms, c->ev[6], c->ev[7]) == cudaSuccess) c->st.t_lattice_ms = ms;
-  if (st[0] | st[1]) return status_to_code(c, st[0] | st[1]);
+  if (st) return status_to_code(c, st);
   return PEPCG_OK;
 }
 
