@@ -303,8 +303,15 @@ constexpr size_t walk_block_smem() {
          4 * 64 * sizeof(double);
 }
 
+// Resident blocks per SM: 1 of sixteen warps, 2 of eight; five of four warps where 96
+// registers do (the default form: 200,003 particles 1.69 -> 1.60 ms against four blocks).
 template <int W, bool kStrict>
-__global__ void __launch_bounds__(32 * W, W == 16 ? 1 : (W == 8 ? 2 : 4))
+constexpr int walk_block_resident() {
+  return W == 16 ? 1 : W == 8 ? 2 : kStrict ? 4 : 5;
+}
+
+template <int W, bool kStrict>
+__global__ void __launch_bounds__(32 * W, walk_block_resident<W, kStrict>())
     k_walk_block64(MixArgs A, int* __restrict__ gstack, int nparts, int sweep) {
   constexpr int kThreads = 32 * W;
   constexpr int kRingB = 2 * kThreads;
@@ -590,20 +597,19 @@ bool launch_block(Ctx* c, K kern, int threads, size_t smem, int blocks, int npar
 
 }  // namespace
 
-// Measured when the choice was made (walk ms, Plummer, theta 0.4, one warp per bucket ->
-// the choice here; both are some per cent faster since):
-// 16 buckets 0.182 -> 0.044, 64: 0.48 -> 0.064, 141: 0.74 -> 0.114, 257: 1.04 -> 0.21,
-// 516: 1.29 -> 0.36, 938: 1.44 -> 0.59, 1,563: 1.60 -> 0.92, 3,126: 1.83 -> 1.78, and past
-// that one warp per bucket is faster (6,250: 3.48 against 3.62).  Eight warps at two blocks
-// per SM beat sixteen except for 75 .. 148 buckets, which leave an SM one block each
-// (141 buckets: 0.114 against 0.137 in clusters of two); four warps from 600 buckets on
-// (516: 0.38 against 0.36, 938: 0.59 against 0.62).  The adjoint's records carry
-// more arithmetic per round, so its line lies higher (4,688 buckets: 6.2 against 6.7 ms).
+// Measured (walk ms, Plummer, theta 0.4, one warp per bucket -> the choice here):
+// 16 buckets 0.182 -> 0.042, 64: 0.48 -> 0.064, 141: 0.74 -> 0.114, 257: 1.10 -> 0.20,
+// 516: 1.31 -> 0.33, 938: 1.42 -> 0.52, 1,563: 1.54 -> 0.86, 3,126: 1.77 -> 1.60, 6,250:
+// 3.42 -> 3.24, and past that one warp per bucket is faster (12,500: 6.46 against 6.56;
+// strict: 3,126: 2.48 -> 2.24, 6,250 level).  Eight warps at two blocks per SM beat sixteen
+// except for 75 .. 148 buckets, which leave an SM one block each (141 buckets: 0.114
+// against 0.137 in clusters of two); four warps from 600 buckets on (516: 0.37 against
+// 0.33, 938: 0.52 against 0.58).  The adjoint: 4,688 buckets 6.2 against 6.7 ms.
 // Few buckets on a large tree are scattered targets with long lists: sixteen warps
 // and eight blocks (8 buckets, 262,144 sources: 0.135 against 0.18 ms).
-bool block_walk_shape(int64_t nt, int64_t npart, bool adjoint, BlockShape* sh) {
+bool block_walk_shape(int64_t nt, int64_t npart, BlockWalk kind, BlockShape* sh) {
   const int64_t nb = (nt + 63) / 64;
-  if (nb > (adjoint ? 6000 : 3200)) return false;
+  if (nb > (kind == BlockWalk::kStrict ? 5000 : kind == BlockWalk::kAdjoint ? 6000 : 9000)) return false;
   if (nb <= 18 && npart >= 32768) *sh = {16, 8};
   else if (nb <= 37) *sh = {8, 8};
   else if (nb <= 74) *sh = {8, 4};
@@ -614,17 +620,18 @@ bool block_walk_shape(int64_t nt, int64_t npart, bool adjoint, BlockShape* sh) {
 }
 
 // One cluster per bucket, or resident blocks that take buckets from the queue.
-static int block_grid(const BlockShape& sh, int64_t nt) {
+static int block_grid(const BlockShape& sh, int64_t nt, int per_sm) {
   const int64_t nb = (nt + 63) / 64;
   if (sh.parts > 1) return (int)(nb * sh.parts);
-  return (int)std::min<int64_t>(nb, sh.warps == 16 ? 148 : sh.warps == 8 ? 296 : 592);
+  return (int)std::min<int64_t>(nb, 148 * per_sm);
 }
 
 bool launch_walk_block64(Ctx* c, const MixArgs& A, const BlockShape& sh, bool strict, int* stack,
                          cudaStream_t s) {
   const int sweep = (!strict && A.M <= (1 << kBoxShift)) ? A.nbox : 1;
   auto go = [&](auto kern, int W, size_t smem) {
-    return launch_block(c, kern, 32 * W, smem, block_grid(sh, A.nt), sh.parts, s, A, stack, sweep);
+    const int per_sm = W == 16 ? 1 : W == 8 ? 2 : strict ? 4 : 5;
+    return launch_block(c, kern, 32 * W, smem, block_grid(sh, A.nt, per_sm), sh.parts, s, A, stack, sweep);
   };
   if (sh.warps == 16)
     return strict ? go(k_walk_block64<16, true>, 16, walk_block_smem<16, true>())
@@ -640,7 +647,8 @@ bool launch_adj_block64(Ctx* c, const AdjMixArgs& A, const BlockShape& sh, bool 
                         cudaStream_t s) {
   const int sweep = c->nnodes <= (1 << kBoxShift) ? A.nbox : 1;
   auto go = [&](auto kern, int W, size_t smem) {
-    return launch_block(c, kern, 32 * W, smem, block_grid(sh, A.nt), sh.parts, s, A, stack, sweep);
+    const int per_sm = W == 16 ? 1 : W == 8 ? 2 : 4;
+    return launch_block(c, kern, 32 * W, smem, block_grid(sh, A.nt, per_sm), sh.parts, s, A, stack, sweep);
   };
   if (sh.warps == 16)
     return with_e ? go(k_adj_block64<16, true>, 16, adj_block_smem<16, true>())

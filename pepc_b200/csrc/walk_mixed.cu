@@ -1071,11 +1071,11 @@ int launch_walk_mixed(Ctx* c, int64_t nt, const double* tx, const double* ty, co
   A.npacks = npacks;
   BlockShape sh;
   const bool group64 = !per_target && !tflag && tiles == nullptr && c->group_size() == 64;
-  if (group64 && block_walk_shape(shape_nt, c->n, false, &sh)) {
+  const bool strict = c->prm.precision == PEPCG_PRECISION_MIXED_STRICT;
+  if (group64 && block_walk_shape(shape_nt, c->n, strict ? BlockWalk::kStrict : BlockWalk::kDefault, &sh)) {
     const size_t per = (size_t)148 * 5 * kWW * kStackCap;
     if (!ensure(c, c->wstack, 2 * per, "walk stacks")) return PEPCG_ERR_OOM;
-    return launch_walk_block64(c, A, sh, c->prm.precision == PEPCG_PRECISION_MIXED_STRICT,
-                               c->wstack.p + slot * per, s) ? PEPCG_OK : PEPCG_ERR_CUDA;
+    return launch_walk_block64(c, A, sh, strict, c->wstack.p + slot * per, s) ? PEPCG_OK : PEPCG_ERR_CUDA;
   }
   COUNT_LAUNCH();
   if (per_target) {
@@ -1133,7 +1133,7 @@ int launch_adjoint_group64(Ctx* c, int64_t nt, const double* tx, const double* t
   const size_t per = (size_t)gblocks * kWW * kStackCap;
   if (!ensure(c, c->wstack, 2 * per, "walk stacks")) return PEPCG_ERR_OOM;
   BlockShape sh;
-  if (block_walk_shape(nt, c->n, true, &sh))
+  if (block_walk_shape(nt, c->n, BlockWalk::kAdjoint, &sh))
     return launch_adj_block64(c, A, sh, with_e, c->wstack.p, s) ? PEPCG_OK : PEPCG_ERR_CUDA;
   COUNT_LAUNCH();
   if (with_e)

@@ -16,7 +16,7 @@ import pepc_b200 as P
 pytestmark = pytest.mark.gpu
 
 EDGES = [1, 63, 64, 65, 18 * 64, 18 * 64 + 1, 37 * 64, 37 * 64 + 1, 74 * 64, 74 * 64 + 1, 148 * 64,
-         148 * 64 + 1, 600 * 64 + 1, 3200 * 64 + 1]
+         148 * 64 + 1, 600 * 64 + 1, 5000 * 64 + 1, 9000 * 64 + 1]
 
 
 def sources(n, seed):
