@@ -689,7 +689,7 @@ bool downward_pass(Ctx* c, cudaStream_t s) {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     if (cudaLaunchKernelEx(&cfg, k_adj_down, 0, c->max_level - 1, D, c->barrier_word(2),
-                           c->d_status + 1) == cudaSuccess) {
+                           c->d_tree_status) == cudaSuccess) {
       COUNT_LAUNCH();
       return true;
     }

@@ -357,15 +357,12 @@ int pepcg_create(void** out, const pepcg_params* p) {
     pepcg_destroy(c);
     return PEPCG_ERR_CUDA;
   }
-  c->d_status = reinterpret_cast<uint32_t*>(c->d_small + 32);
+  c->counters = c->d_small + 12;
+  c->d_status = reinterpret_cast<uint32_t*>(c->d_small + 20);
+  c->d_tree_status = reinterpret_cast<uint32_t*>(c->d_small + 21);
   c->lvlcnt = reinterpret_cast<int32_t*>(c->d_small + 34);
   prepare_boxes(c);
   cudaMemcpy(c->d_vbox, c->vbox, 3 * c->nboxes * sizeof(double), cudaMemcpyHostToDevice);
-  if (!ensure(c, c->counters, 8, "counters")) {
-    g_static_err = c->err;
-    pepcg_destroy(c);
-    return PEPCG_ERR_OOM;
-  }
   if (c->far_field) {
     rc = lattice_prepare(c);
     if (rc) {
@@ -398,7 +395,7 @@ int pepcg_destroy(void* ctx) {
   release(c->tinfo); release(c->tcounts); release(c->macb); release(c->first_part);
   release(c->nleaves); release(c->child8); release(c->wstack); release(c->over); release(c->leafnode);
   release(c->adj); release(c->fpo2rpo); release(c->rpo2fpo); release(c->nkey);
-  release(c->tiles); release(c->counters); release(c->tgt); release(c->tkeys);
+  release(c->tiles); release(c->tgt); release(c->tkeys);
   for (void* p : {(void*)c->d_box, (void*)c->d_small, (void*)c->d_vbox,
                   (void*)c->d_part, (void*)c->d_mlattice, (void*)c->d_lattab, (void*)c->d_latcoef,
                   (void*)c->d_latpart, (void*)c->d_ofict, (void*)c->d_site, (void*)c->d_site_q,

@@ -415,6 +415,30 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T* smem, T& total) {
   return wpre + x - v;
 }
 
+// The values the host needs before the rest of the tree can be launched, into mapped
+// host memory: the node starts of the last particle (scanned and its own, their sum is
+// the node count), box and boxlength2, the duplicate count, the deepest leaf level,
+// twigs per level and the status word.  By one block, or by the last block of the scan.
+struct SummaryArgs {
+  const double* box;
+  const unsigned long long* small;
+  const uint32_t* status;
+  const int32_t* lvl;
+  Ctx::GrowSummary* out;  // nullptr: no summary
+};
+__device__ __forceinline__ void grow_summary(const SummaryArgs& A, int32_t before_last, int32_t last) {
+  const int t = threadIdx.x;
+  if (t < 9 + kMaxLevel + 1) A.out->box[t] = A.box[t];
+  if (t <= kMaxLevel) A.out->lvl[t] = A.lvl[t];
+  if (t == 0) {
+    A.out->dup_count = A.small[0];
+    A.out->starts_before_last = before_last;
+    A.out->starts_last = last;
+    A.out->status = *A.status;
+    A.out->max_level = *reinterpret_cast<const int*>(A.small + 2);
+  }
+}
+
 // One or two arrays of the same length per launch (blockIdx.y picks the
 // array); block sums at bsum[blockIdx.y * gridDim.x + blockIdx.x].
 template <class T>
@@ -500,7 +524,8 @@ __global__ void k_scan_apply(ScanPair<T> a, int64_t n, const T* __restrict__ bsu
 // three paired scans of 16,411 particles take 16 us instead of 22 (ncu).
 template <class T>
 __global__ void __launch_bounds__(kThreads) k_scan_coop(ScanPair<T> a, int64_t n, T* bsum,
-                                                        unsigned* word, uint32_t* status) {
+                                                        unsigned* word, uint32_t* status,
+                                                        SummaryArgs S) {
   __shared__ T sm[32];
   const int64_t base = (int64_t)blockIdx.x * kScanTile;
   const T* in = blockIdx.y ? a.in[1] : a.in[0];
@@ -526,8 +551,21 @@ __global__ void __launch_bounds__(kThreads) k_scan_coop(ScanPair<T> a, int64_t n
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     if (i0 + k < n) out[i0 + k] = ex;
+    if (S.out && i0 + k == n - 1) {  // the last element's prefix and value
+      sm[0] = ex;
+      sm[1] = v[k];
+    }
     ex += v[k];
   }
+  if (S.out && blockIdx.y == 0 && blockIdx.x == gridDim.x - 1) {
+    __syncthreads();
+    grow_summary(S, (int32_t)sm[0], (int32_t)sm[1]);
+  }
+}
+
+__global__ void k_grow_summary(int64_t n, const int32_t* __restrict__ sstart,
+                               const int32_t* __restrict__ cstart, SummaryArgs S) {
+  grow_summary(S, sstart[n - 1], cstart[n - 1]);
 }
 
 // exclusive scans of one array, or of two arrays of the same length in the
@@ -535,7 +573,8 @@ __global__ void __launch_bounds__(kThreads) k_scan_coop(ScanPair<T> a, int64_t n
 // zeroed barrier word and the status word that let small arrays take one launch
 template <class T>
 void exclusive_scan2(const T* in0, T* out0, const T* in1, T* out1, int64_t n, T* tmp,
-                     cudaStream_t s, unsigned* word = nullptr, uint32_t* status = nullptr) {
+                     cudaStream_t s, unsigned* word = nullptr, uint32_t* status = nullptr,
+                     const SummaryArgs& sum = SummaryArgs{}) {
   const int64_t nb = (n + kScanTile - 1) / kScanTile;
   ScanPair<T> a{{in0, in1}, {out0, out1}};
   const dim3 grid((unsigned)nb, in1 ? 2u : 1u);
@@ -549,7 +588,7 @@ void exclusive_scan2(const T* in0, T* out0, const T* in1, T* out1, int64_t n, T*
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_scan_coop<T>, a, n, tmp, word, status) == cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, k_scan_coop<T>, a, n, tmp, word, status, sum) == cudaSuccess) {
       COUNT_LAUNCH();
       return;
     }
@@ -559,6 +598,11 @@ void exclusive_scan2(const T* in0, T* out0, const T* in1, T* out1, int64_t n, T*
   k_scan_reduce<T><<<grid, kThreads, 0, s>>>(a, n, tmp);
   COUNT_LAUNCH();
   k_scan_apply<T><<<grid, kThreads, 0, s>>>(a, n, tmp);
+  if (sum.out) {
+    COUNT_LAUNCH();
+    k_grow_summary<<<1, 64, 0, s>>>(n, reinterpret_cast<const int32_t*>(out0),
+                                    reinterpret_cast<const int32_t*>(in0), sum);
+  }
 }
 
 template <class T>
@@ -969,27 +1013,6 @@ __global__ void k_node_counts(int64_t n, const int64_t* __restrict__ key,
   __syncthreads();
   if (threadIdx.x == 0 && bmax > 0) atomicMax(maxlev, bmax);
   if (threadIdx.x <= kMaxLevel && h[threadIdx.x]) atomicAdd(&lvl[threadIdx.x], h[threadIdx.x]);
-}
-
-// The values the host needs before the rest of the tree can be launched,
-// into mapped host memory: the node starts of the last particle (scanned and
-// its own, their sum is the node count), box and boxlength2, the duplicate
-// count, the deepest leaf level, twigs per level and the status word.
-__global__ void k_grow_summary(int64_t n, const int32_t* __restrict__ sstart,
-                               const int32_t* __restrict__ cstart, const double* __restrict__ box,
-                               const unsigned long long* __restrict__ small,
-                               const uint32_t* __restrict__ status,
-                               const int32_t* __restrict__ lvl, Ctx::GrowSummary* out) {
-  const int t = threadIdx.x;
-  if (t < 9 + kMaxLevel + 1) out->box[t] = box[t];
-  if (t <= kMaxLevel) out->lvl[t] = lvl[t];
-  if (t == 0) {
-    out->dup_count = small[0];
-    out->starts_before_last = sstart[n - 1];
-    out->starts_last = cstart[n - 1];
-    out->status = *status;
-    out->max_level = *reinterpret_cast<const int*>(small + 2);
-  }
 }
 
 // Largest j >= from with key[j] >> sh == prefix (key[from] is known to match).
@@ -1839,7 +1862,7 @@ static void upward_pass(Ctx* c, const UpArgs& U, cudaStream_t s) {
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_upward_all, c->max_level - 1, U, c->barrier_word(1), c->d_status + 1) ==
+    if (cudaLaunchKernelEx(&cfg, k_upward_all, c->max_level - 1, U, c->barrier_word(1), c->d_tree_status) ==
         cudaSuccess) {
       COUNT_LAUNCH();
       return;
@@ -1930,13 +1953,12 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
                                                   c->cend.p, c->d_status,
                                                   reinterpret_cast<int*>(c->d_small + 2),
                                                   c->lvlcnt);
+  c->h_sum->status = ST_TIMEOUT;  // what stands if the scan's barrier gives up
+  // the host needs the node count M (grid sizes, allocations), the box, the level
+  // counts and the status: the scan's last block writes them to mapped host memory
   exclusive_scan2<int32_t>(c->cstart.p, c->sstart.p, c->cend.p, c->send.p, n, c->scan_tmp.p, s,
-                           c->barrier_word(4), c->d_status);
-  // the host needs the node count M (grid sizes, allocations), the box, the
-  // level counts and the status: one kernel writes them to mapped host memory
-  COUNT_LAUNCH();
-  k_grow_summary<<<1, 64, 0, s>>>(n, c->sstart.p, c->cstart.p, c->d_box, c->d_small, c->d_status,
-                                  c->lvlcnt, c->d_sum);
+                           c->barrier_word(4), c->d_status,
+                           SummaryArgs{c->d_box, c->d_small, c->d_status, c->lvlcnt, c->d_sum});
   if (!cuda_ok(c, cudaEventRecord(c->sum_ev, s), "grow summary")) return PEPCG_ERR_CUDA;
   cudaEventRecord(c->ev[9], s);
   // the particles into key order run while the host waits for the summary
@@ -2005,7 +2027,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
   // count; the deepest twig level is one above the deepest leaf level
   {
     exclusive_scan2<int32_t>(bt, bt, ba, ba, (int64_t)nlb, c->scan_tmp.p, s, c->barrier_word(5),
-                             c->d_status + 1);
+                             c->d_tree_status);
     COUNT_LAUNCH();
     int32_t* cc = c->tcounts.p;
     int32_t* tcn = c->tcounts.p + ntw;
@@ -2013,7 +2035,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
                                             c->nc4.p, c->drec.p, c->lvlpos.p, c->child8.p,
                                             c->nchild.p, c->tinfo.p, cc, tcn);
     exclusive_scan2<int32_t>(cc, cc, tcn, tcn, ntw, c->scan_tmp.p, s, c->barrier_word(6),
-                             c->d_status + 1);
+                             c->d_tree_status);
     UpArgs U{c->lvlcnt, c->twiglist.p, c->tinfo.p, cc, tcn, c->nleaves.p, c->drec.p,
              c->dmom.p, c->nc4.p, c->mom.p, reinterpret_cast<float4*>(c->mom32.p)};
     upward_pass(c, U, s);

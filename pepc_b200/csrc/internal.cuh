@@ -191,20 +191,21 @@ struct Ctx {
   DBuf<int64_t> nkey;
   // walk scratch
   DBuf<int32_t> tiles;        // PER_TILE tile boundaries
-  DBuf<unsigned long long> counters;  // interaction counters
   DBuf<double> tgt;           // staging for host targets / results
   DBuf<int64_t> tkeys;
   // small device state: box (9), boxlength2 (21), status word, dup count ...
   double* d_box = nullptr;    // [0..8] box, [9..29] boxlength2
-  // status words: [0] of the running call, [1] of the tree's later kernels (upward pass,
-  // adjoint), which nothing waits for: read with the next walk's status
+  // status words: of the running call, and (d_tree_status) of the tree's later kernels
+  // (upward pass, adjoint), which nothing waits for: read with the next walk's status
   uint32_t* d_status = nullptr;
-  unsigned long long* d_small = nullptr;  // [0] dup count, [1] nnodes, [2] tile count, ...
-                                          // [8], [9] walk bucket queues (one per walk
-                                          // stream), [10] adjoint item queue,
-                                          // [16] .. [19] grid barriers and block
-                                          // counters (32-bit words); then d_status
-                                          // and lvlcnt, so that one memset clears all
+  // [0] dup count, [1] nnodes, [2] tile count, ...; [8], [9] walk bucket queues (one per
+  // walk stream), [10] adjoint item queue, [11] equal pairs, [12] .. [15] interaction
+  // counters, [16] .. [19] grid barriers and block counters (32-bit words), [20]
+  // d_status, [21] d_tree_status, [34] .. lvlcnt: one memset clears all for a grow,
+  // one clears [8, 21) for a walk
+  unsigned long long* d_small = nullptr;
+  unsigned long long* counters = nullptr;
+  uint32_t* d_tree_status = nullptr;
   static constexpr int kSmall = 34 + 16;
   double box[9];
   double boxlength2[kMaxLevel + 1];

@@ -1059,7 +1059,7 @@ int launch_walk_mixed(Ctx* c, int64_t nt, const double* tx, const double* ty, co
   A.M = (int32_t)c->nnodes;
   A.npart = c->n;
   A.ex = ex; A.ey = ey; A.ez = ez; A.pot = pot; A.work = work;
-  A.counters = c->counters.p;
+  A.counters = c->counters;
   A.status = c->d_status;
   A.queue = c->walk_queue(slot);
   A.tiles = tiles;
@@ -1126,7 +1126,7 @@ int launch_adjoint_group64(Ctx* c, int64_t nt, const double* tx, const double* t
   A.eps2 = (float)c->prm.eps2;
   A.npart = c->n;
   A.adj = c->adj.p;
-  A.counters = c->counters.p;
+  A.counters = c->counters;
   A.status = c->d_status;
   A.queue = c->walk_queue();
   const int gblocks = 148 * 4;

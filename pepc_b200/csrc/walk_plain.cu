@@ -918,9 +918,10 @@ static int list_bucket(int64_t nt) {
 // device-to-host copies to pageable memory and their staging took 10 us more).
 static __global__ void k_walk_summary(const unsigned long long* __restrict__ ctr,
                                       const uint32_t* __restrict__ status,
+                                      const uint32_t* __restrict__ tree_status,
                                       const int32_t* __restrict__ over, Ctx::GrowSummary* out) {
   if (threadIdx.x < 3) out->ctr[threadIdx.x] = ctr[threadIdx.x];
-  if (threadIdx.x == 3) out->walk_status = status[0] | status[1];  // see Ctx::d_status
+  if (threadIdx.x == 3) out->walk_status = *status | *tree_status;
   if (threadIdx.x == 4) out->nover = over ? *over : 0;
 }
 
@@ -941,8 +942,8 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   }
   cudaStream_t s = c->stream;
   const int walk = c->prm.walk;
-  if (!cuda_ok(c, cudaMemsetAsync(c->counters.p, 0, 4 * sizeof(unsigned long long), s), "ctr") ||
-      !cuda_ok(c, cudaMemsetAsync(c->d_status, 0, 4, s), "status"))
+  // bucket queues, counters, barrier words and the status word
+  if (!cuda_ok(c, cudaMemsetAsync(c->d_small + 8, 0, 13 * sizeof(unsigned long long), s), "walk state"))
     return PEPCG_ERR_CUDA;
   int64_t ntiles = 0;
   if (walk == PEPCG_WALK_PER_TILE) {
@@ -1044,7 +1045,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   A.eps2 = c->prm.eps2;
   A.M = (int32_t)c->nnodes;
   A.npart = c->n;
-  A.counters = c->counters.p;
+  A.counters = c->counters;
   A.status = c->d_status;
   A.queue = c->walk_queue();
   A.tiles = reinterpret_cast<const int2*>(c->tiles.p);
@@ -1094,8 +1095,10 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
       A.tx = tx + t0; A.ty = ty + t0; A.tz = tz + t0;
       A.ex = ex + t0; A.ey = ey + t0; A.ez = ez + t0; A.pot = pot + t0; A.work = work + t0;
       A.tq = tq ? tq + t0 : nullptr;
-      COUNT_LAUNCH();
-      k_reset_counter<<<1, 1, 0, sk>>>(A.queue);
+      if (k >= 2) {  // a chunk's queue again (the first two are zero)
+        COUNT_LAUNCH();
+        k_reset_counter<<<1, 1, 0, sk>>>(A.queue);
+      }
       if (c->prm.precision == PEPCG_PRECISION_PLAIN) {
         COUNT_LAUNCH();
         const int law = c->prm.force_law;
@@ -1149,7 +1152,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   if (plan && plan->before_sync && !plan->before_sync()) return PEPCG_ERR_CUDA;
   auto summary = [&]() {
     COUNT_LAUNCH();
-    k_walk_summary<<<1, 32, 0, s>>>(c->counters.p, c->d_status, lists ? c->over.p : nullptr, c->d_sum);
+    k_walk_summary<<<1, 32, 0, s>>>(c->counters, c->d_status, c->d_tree_status, lists ? c->over.p : nullptr, c->d_sum);
     return cuda_ok(c, cudaGetLastError(), "walk summary") &&
            cuda_ok(c, cudaStreamSynchronize(s), "walk");
   };
