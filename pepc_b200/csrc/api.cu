@@ -695,7 +695,8 @@ int pepcg_traverse_tree(void* ctx, int64_t nt, const double* tx, const double* t
   const double* tq =
       c->prm.force_law == 5 ? grown_charges_if_same(c, nt, keys_used ? c->tkeys.p : nullptr) : nullptr;
   int rc = traverse_device(c, nt, b, b + nt, b + 2 * nt, keys_used ? c->tkeys.p : nullptr, false,
-                           b + 3 * nt, b + 4 * nt, b + 5 * nt, b + 6 * nt, b + 7 * nt, tq);
+                           b + 3 * nt, b + 4 * nt, b + 5 * nt, b + 6 * nt, b + 7 * nt, tq, nullptr, 0,
+                           tkeys != nullptr);
   if (rc && rc != PEPCG_WARN_NOT_NEUTRAL) return rc;
   for (int k = 0; k < 5; ++k)
     ok = ok && cuda_ok(c, cudaMemcpyAsync(hout[k], b + (3 + k) * nt, nt * 8, cudaMemcpyDeviceToHost, s), "D2H");

@@ -376,6 +376,9 @@ int host_tiles(Ctx* c, int64_t nt, const int64_t* d_tkeys, int T, int2* d_tiles,
 // shape_nt: the target count by which the mixed group walk picks its kernel
 // (0: nt).  Chunks and ranges of one target set pass the whole set's count, so
 // that the split does not change a bucket's sums.
+//
+// keyed: the caller has the targets' keys (tkeys, or keys that this walk does not
+// read), so they lie in key order.
 struct ChunkPlan {
   int nchunks = 1;
   const int64_t* bounds = nullptr;  // nchunks + 1 target offsets
@@ -386,7 +389,7 @@ struct ChunkPlan {
 int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const double* tz,
                     const int64_t* tkeys, bool self, double* ex, double* ey, double* ez,
                     double* pot, double* work, const double* tq = nullptr,
-                    const ChunkPlan* plan = nullptr, int64_t shape_nt = 0);
+                    const ChunkPlan* plan = nullptr, int64_t shape_nt = 0, bool keyed = false);
 
 // walk_mixed.cu: the transposed adjoint walk of the mixed 64-target group walk
 int launch_adjoint_group64(Ctx* c, int64_t nt, const double* tx, const double* ty,

@@ -69,8 +69,8 @@ struct WalkArgs {
   const int32_t* fpo2rpo;
   uint2* lstack;       // kListStack entries per resident block
   int lper;            // per target: targets per bucket (8, 16 or 32)
-  // buckets (packs) whose lists did not fit: [0] their number, then their indices.
-  // Written by k_walk_list64; k_walk_target64 / k_walk_tilepack64 walk them (kOnly)
+  // what k_walk_list64 left to k_walk_target64 / k_walk_tilepack64 (kOnly): [0] their
+  // number, then targets (count << 20 | first) or packs
   int32_t* over;
 };
 
@@ -97,7 +97,9 @@ __device__ __forceinline__ void warp_add_counters(unsigned long long* ctr, unsig
   }
 }
 
-// kOnly: walks the buckets that A.over lists (a separate instantiation: the test inside
+constexpr int kOverShift = 20;
+
+// kOnly: walks the targets that A.over lists (a separate instantiation: the test inside
 // the queue loop cost the walk of 250,000 targets 10 %)
 template <int kLaw, bool kCut, bool kOnly = false>
 __global__ void __launch_bounds__(kWalkThreads) k_walk_target64(WalkArgs A) {
@@ -113,13 +115,16 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_target64(WalkArgs A) {
     unsigned b = 0;
     if (lane == 0) b = atomicAdd(A.queue, 1u);
     b = __shfl_sync(0xffffffffu, b, 0);
+    int64_t t0 = (int64_t)b * 32;
+    int per = 32;
     if constexpr (kOnly) {
       if ((int)b >= A.over[0]) break;
-      b = (unsigned)A.over[1 + b];
+      const int o = A.over[1 + b];
+      t0 = o & ((1 << kOverShift) - 1);
+      per = o >> kOverShift;
     }
-    const int per = kOnly ? A.lper : 32;
-    if ((int64_t)b * per >= A.nt) break;
-    const int64_t t = (int64_t)b * per + lane;
+    if (t0 >= A.nt) break;
+    const int64_t t = t0 + lane;
     const bool valid = t < A.nt && (!kOnly || lane < per);
     double px = 0, py = 0, pz = 0, e0 = 0, e1 = 0, e2 = 0, ph = 0, w = 0;
     KelbgArgs kel{0.0, A.kinv, A.sqrtpi};
@@ -447,8 +452,13 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_walk_tilepack64(WalkArgs A)
 // The walks above give a bucket to one warp, a serial chain of dependent loads and FP64
 // latencies (4,099 particles are 129 such warps), and evaluate with 77 % of the lanes
 // active (here 96 %).
-// Lists hold kListCap entries (shared memory: two blocks per SM); a longer
-// one is left to the walks above (A.over).
+// Lists hold kListCap entries (shared memory: two blocks per SM).  Where scattered
+// targets' union is longer, the per-target walk goes on with half as many targets, down
+// to kListMin (a target's result does not depend on its bucket); what is still
+// too long, and a pack, is left to the walks above (A.over), and so are the block's next 1, 2, 4,
+// .. 16 buckets unsearched while this goes on.  16,000 of 100,000 uniform particles in any
+// order, theta 0.4: 18.3 ms by warps, 19.0 with whole buckets left to them, 7.0 so; 1,000 of
+// 1M Plummer particles, of which four are often too many: 31.1 / 16.7 / 16.3.
 constexpr int kListThreads = 256;
 constexpr int kListWarps = kListThreads / 32;
 constexpr int kListCap = 8192;
@@ -457,6 +467,7 @@ constexpr int kListPop = kListWarps * kListNodes;
 // a pop takes at most kListPop entries and each pushes at most 8 (one level down)
 constexpr int kListStack = (kMaxLevel + 2) * 8 * kListPop;
 constexpr int kListBatch = 32;  // entries per batch
+constexpr int kListMin = 4;     // targets
 
 struct __align__(16) ListShared {
   unsigned long long list[kListCap];            // order index << 33 | leaf << 32 | target mask
@@ -481,14 +492,30 @@ __global__ void __launch_bounds__(kListThreads, 2) k_walk_list64(WalkArgs A) {
   const int64_t nbk = kTile ? (int64_t)*A.npacks : (A.nt + A.lper - 1) / A.lper;
   const double vx = A.vbox[0], vy = A.vbox[1], vz = A.vbox[2];
   unsigned long long c_leaf = 0, c_twig = 0, c_mac = 0;
+  int64_t b = 0, first = 0;  // bucket, and its targets [first, first + left) to do (per target)
+  int left = 0;
+  int width = kTile ? 32 : A.lper, fits = 0;  // targets at a time, lists in a row that fitted
+  int back = 0, skip = 0;                     // buckets to leave unsearched: after a miss, now
   for (;;) {
-    if (tid == 0) S.bucket = atomicAdd(A.queue, 1u);
+    if (left == 0) {
+      if (tid == 0) S.bucket = atomicAdd(A.queue, 1u);
+      __syncthreads();
+      b = S.bucket;
+      if (b >= nbk) break;
+      first = b * A.lper;
+      left = kTile ? 1 : (int)min((int64_t)A.lper, A.nt - first);
+      if (skip > 0) {
+        --skip;
+        if (tid == 0) A.over[1 + atomicAdd(A.over, 1)] = kTile ? (int32_t)b : left << kOverShift | (int32_t)first;
+        left = 0;
+        __syncthreads();
+        continue;
+      }
+    }
     if (tid < 32) S.partner[tid] = 0u;
-    __syncthreads();
-    const int64_t b = S.bucket;
-    if (b >= nbk) break;
     bool valid;
     int64_t t0;
+    const int len = min(width, left);
     unsigned tmask = 0u;  // the lanes of this lane's tile
     if (kTile) {
       int tl0, len;
@@ -496,12 +523,13 @@ __global__ void __launch_bounds__(kListThreads, 2) k_walk_list64(WalkArgs A) {
       valid = pack_lane(A.pstart, A.tflag, b, lane, tl0, len);
       tmask = valid ? (((len >= 32) ? 0xffffffffu : ((1u << len) - 1u)) << tl0) : 0u;
     } else {
-      t0 = b * A.lper;
-      valid = lane < A.lper && t0 + lane < A.nt;
+      t0 = first;
+      valid = lane < len;
     }
     const unsigned all = __ballot_sync(0xffffffffu, valid);
     if (all == 0u) {
       if (tid == 0) atomicOr(A.status, ST_INCOMPLETE);  // a pack must start with a tile
+      left = 0;
       __syncthreads();
       continue;
     }
@@ -616,10 +644,22 @@ __global__ void __launch_bounds__(kListThreads, 2) k_walk_list64(WalkArgs A) {
       __syncthreads();
     }
     if (over) {
-      if (tid == 0) A.over[1 + atomicAdd(A.over, 1)] = (int32_t)b;
+      fits = 0;
+      if (!kTile && len > kListMin) {
+        width = max(len >> 1, kListMin);
+      } else {
+        if (tid == 0) A.over[1 + atomicAdd(A.over, 1)] = kTile ? (int32_t)b : left << kOverShift | (int32_t)first;
+        left = 0;
+        skip = back = min(16, max(1, 2 * back));
+      }
       __syncthreads();
       continue;
     }
+    back = 0;
+    left -= len;
+    first += len;
+    if (kTile) left = 0;
+    else if (++fits >= 16 && width < A.lper) fits = 0, width = min(2 * width, A.lper);
     c_mac += mac;
     atomicAdd(&S.partner[lane], partner);
     // ---- 2. node order: bitonic sort, padded to a power of two
@@ -894,15 +934,20 @@ int prepare_mac(Ctx* c, const double** macb) {
 // 1.10 -> 0.69.  With more buckets the lists' own work (sort, packing, a
 // node per warp step in the search: 480 instructions per 32 interactions, 158 of them
 // FP64) costs more than idle lanes: 100,003: 3.04 against 3.43, 250,000: 6.4 against 9.0.
+// Targets without keys may lie in any order: their line is lower, since scattered targets
+// share few nodes (theta 0.4, of 100,000 Plummer particles: 4,000 targets 20.0 -> 4.1, 16,000:
+// 24.0 -> 14.0, in proportion from there on, against 24.5 by warps for 64,000; on a line
+// through them 64,000 targets 3.9 by warps, 4.4 by lists).
 constexpr int64_t kListTargets = 65536;
+constexpr int64_t kListOthers = 24576;
 constexpr int kListBlocks = 148 * 2;
-static bool use_list_walk(const Ctx* c, int64_t nt, bool chunked, bool packed) {
+static bool use_list_walk(const Ctx* c, int64_t nt, bool keyed, bool chunked, bool packed) {
   const pepcg_params& p = c->prm;
   if (p.precision != PEPCG_PRECISION_PLAIN || chunked || p.force_law != 3 || has_spatial_cutoff(p) ||
       c->nboxes != 1)
     return false;
   if (p.walk != PEPCG_WALK_PER_TARGET && !packed) return false;
-  if (nt > kListTargets) return false;
+  if (nt > (keyed ? kListTargets : kListOthers)) return false;
   return c->nnodes <= kListCap || (p.mac_select == 0 && p.theta2 >= 0.12);
 }
 
@@ -928,7 +973,7 @@ static __global__ void k_walk_summary(const unsigned long long* __restrict__ ctr
 int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const double* tz,
                     const int64_t* tkeys, bool self, double* ex, double* ey, double* ez,
                     double* pot, double* work, const double* tq, const ChunkPlan* plan,
-                    int64_t shape_nt) {
+                    int64_t shape_nt, bool keyed) {
   if (!c->has_tree) {
     c->err = "traverse called without a grown tree";
     return PEPCG_ERR_NO_TREE;
@@ -1059,13 +1104,13 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   A.has_cut = has_spatial_cutoff(c->prm) ? 1 : 0;
   for (int k = 0; k < 3; ++k) A.cut[k] = c->prm.spatial_interaction_cutoff[k];
   const int blocks = 148 * 8;
-  const bool lists = use_list_walk(c, nt, plan != nullptr, packed);
+  const bool lists = use_list_walk(c, nt, self || tkeys || keyed, plan != nullptr, packed);
   if (lists) {
     A.lper = list_bucket(nt);
     const int64_t nbk = packed ? (nt + kPackChunk - 1) / kPackChunk * kPackSlots
                                : (nt + A.lper - 1) / A.lper;
     if (!ensure(c, c->wstack, (size_t)2 * kListStack * kListBlocks, "walk stacks") ||
-        !ensure(c, c->over, nbk + 1, "walk lists"))
+        !ensure(c, c->over, 1 + (packed ? nbk : (int64_t)nt), "walk lists"))
       return PEPCG_ERR_OOM;
     A.drec = c->drec.p;
     A.rpo2fpo = c->rpo2fpo.p;

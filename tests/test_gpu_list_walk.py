@@ -32,33 +32,41 @@ def both(x, y, z, q, walk, nt=None, shift=0.0, **kw):
 
 
 @pytest.mark.parametrize("walk", [P.WALK_PER_TARGET, P.WALK_PER_TILE])
-@pytest.mark.parametrize("n", [2, 31, 33, 500, 4099, 20011])
+@pytest.mark.parametrize("n", [2, 31, 33, 500, 4099, 20011, 65536, 65537])
 def test_self_fields(gpu, n, walk):
     both(*cube(n, 71, charges="gauss"), walk, theta2=0.36, eps2=1e-6)
 
 
 @pytest.mark.parametrize("walk", [P.WALK_PER_TARGET, P.WALK_PER_TILE])
 def test_lists_that_do_not_fit(gpu, walk):
-    # scattered targets of one bucket on a clustered tree, theta 0.36: some unions of 32
-    # lists are longer than a list, the others are not
-    x, y, z, q = plummer(40000, 72)
+    # a clustered tree, theta 0.36: some unions of 32 lists are longer than a list, the
+    # others are not
+    both(*plummer(40000, 72), walk, theta2=0.13, eps2=1e-6)
+
+
+# buckets of 8, 16 and 32 targets anywhere on a clustered tree, theta 0.36: unions that fit,
+# that fit in parts, and that do not fit with four targets either
+@pytest.mark.parametrize("nt", [3, 1003, 4735, 20011])
+@pytest.mark.parametrize("n", [40000, 200000])
+def test_scattered_targets(gpu, n, nt):
     kw = dict(theta2=0.13, eps2=1e-6)
-    both(x, y, z, q, walk, **kw)
-    if walk == P.WALK_PER_TARGET:
-        tc, orc = P.TreeCode(**kw), O.Oracle(num_threads=8, **kw)
-        tc.pepc_grow_tree(x, y, z, q)
-        orc.grow_tree(x, y, z, q)
-        t = np.random.default_rng(73).permutation(len(x))[:1000]
-        a, b = tc.pepc_traverse_tree(x[t], y[t], z[t]), orc.traverse_tree(x[t], y[t], z[t])
-        for k in KEYS:
-            assert np.array_equal(a[k], b[k]), k
-        tc.close()
-        orc.close()
+    x, y, z, q = plummer(n, 72)
+    tc, orc = P.TreeCode(**kw), O.Oracle(num_threads=8, **kw)
+    tc.pepc_grow_tree(x, y, z, q)
+    orc.grow_tree(x, y, z, q)
+    t = np.random.default_rng(73).permutation(len(x))[:nt]
+    a, b = tc.pepc_traverse_tree(x[t], y[t], z[t]), orc.traverse_tree(x[t], y[t], z[t])
+    for k in KEYS:
+        assert np.array_equal(a[k], b[k]), k
+    st, c = tc.stats(), orc.counters()
+    assert st["interactions"] == c["interactions"]
+    tc.close()
+    orc.close()
 
 
-@pytest.mark.parametrize("nt", [1, 32, 33, 65535, 65536, 65537])
+@pytest.mark.parametrize("nt", [1, 32, 33, 24576, 24577])
 def test_target_counts(gpu, nt):
-    # targets beside the particles, on both sides of the line at 65,536
+    # targets beside the particles, without keys, on both sides of the line at 24,576
     both(*cube(66000, 74), P.WALK_PER_TARGET, nt=nt, shift=1e-3, theta2=0.5, eps2=1e-4)
 
 
