@@ -1106,6 +1106,7 @@ int launch_walk_mixed(Ctx* c, int64_t nt, const double* tx, const double* ty, co
 int launch_adjoint_group64(Ctx* c, int64_t nt, const double* tx, const double* ty,
                            const double* tz, const double* gex, const double* gey,
                            const double* gez, const double* gphi, bool with_e, cudaStream_t s) {
+  if (nt == 0) return PEPCG_OK;  // no records; a grid of no blocks is refused
   AdjMixArgs A;
   A.nt = nt;
   A.tx = tx; A.ty = ty; A.tz = tz;

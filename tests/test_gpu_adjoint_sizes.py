@@ -3,6 +3,7 @@ launch with one block, with many, level by level), by an identity: with the list
 abs_charge-weighted centres fixed under a common factor of the charges, the loss is
 homogeneous of degree one in them, so sum q dL/dq = L.  FP64 walks: 1e-10 of the
 sum of |q dL/dq| (some hundred thousand terms, atomic order)."""
+import numpy as np
 import pytest
 import torch
 
@@ -46,4 +47,20 @@ def test_charges_scale_the_loss(gpu, n):
             fd = (s[0][0] - s[1][0]) / (2 * h)
             scale = o[1 + d].abs().sum()
             assert float((o[1 + d].sum() + fd).abs()) <= 1e-6 * float(scale)
+    tc.close()
+
+
+MODES = [(P.PRECISION_PLAIN, P.WALK_PER_TARGET), (P.PRECISION_PLAIN, P.WALK_PER_TILE),
+         (P.PRECISION_PLAIN, P.WALK_GROUP), (P.PRECISION_MIXED, P.WALK_PER_TARGET),
+         (P.PRECISION_MIXED, P.WALK_GROUP), (P.PRECISION_MIXED_STRICT, P.WALK_GROUP)]
+
+
+@pytest.mark.parametrize("precision,walk", MODES)
+def test_no_targets_give_zero_gradients(gpu, precision, walk):
+    rng = np.random.default_rng(3)
+    none = np.zeros(0)
+    tc = P.TreeCode(theta2=0.25, eps2=1e-4, precision=precision, walk=walk)
+    tc.pepc_grow_tree(*rng.random((3, 500)), rng.standard_normal(500))
+    r = tc.traverse_adjoint(none, none, none, [none] * 3, none, 500)
+    assert all(np.array_equal(r[k], np.zeros(500)) for k in ("q", "x", "y", "z"))
     tc.close()
