@@ -288,6 +288,15 @@ long long pepcg_kernel_launches(void);
  */
 void pepcg_debug_fail_allocations(int64_t after);
 
+/*
+ * pepcg_debug_barrier_tries -- for tests: how often a block of this context's
+ * cooperative kernels looks for the others at a grid barrier before it gives
+ * up (default 2^22, which is also the largest; seconds).  With 0 every
+ * barrier gives up, so the calls that need one return PEPCG_ERR_TIMEOUT, and
+ * the context stays usable.  A negative value restores the default.
+ */
+int pepcg_debug_barrier_tries(void* ctx, int64_t tries);
+
 /* replaces pepc_timber_tree (module_pepc.f90:538 -> module_libpepc_main.f90:129-148) */
 int pepcg_timber_tree(void* ctx);
 int pepcg_stats_get(void* ctx, pepcg_stats* s);

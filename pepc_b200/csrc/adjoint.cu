@@ -569,10 +569,10 @@ __device__ __forceinline__ void adj_down_twig(const DownArgs& D, const DownHead&
   for (int j = 0; j < 7; ++j) a[j] = r[j];
 }
 
-// One level, or (word set) all levels from the root down, a grid barrier between
+// One level, or (cooperative launch) all levels from the root down, a grid barrier between
 // them; the list entries of a group's first twig of the next level are read before it.
 __global__ void __launch_bounds__(kDownThreads) k_adj_down(int level, int last, DownArgs D,
-                                                           unsigned* word, uint32_t* status) {
+                                                           GridBarrier B) {
   __shared__ int s_cnt[kMaxLevel + 1], s_base[kMaxLevel + 1];
   if (threadIdx.x <= kMaxLevel) {
     int base = 0;
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(kDownThreads) k_adj_down(int level, int last, 
     if (level < last) {
       h = down_head(D, s_base[level + 1] + first, first < s_cnt[level + 1]);
       if (gridDim.x > 1) {
-        if (!grid_barrier(word, ++barriers * gridDim.x, status)) return;
+        if (!grid_barrier(B, ++barriers * gridDim.x)) return;
       } else {
         __syncthreads();
       }
@@ -688,8 +688,8 @@ bool downward_pass(Ctx* c, cudaStream_t s) {
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_adj_down, 0, c->max_level - 1, D, c->barrier_word(2),
-                           c->d_tree_status) == cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, k_adj_down, 0, c->max_level - 1, D,
+                           c->barrier(2, c->d_tree_status)) == cudaSuccess) {
       COUNT_LAUNCH();
       return true;
     }
@@ -700,7 +700,7 @@ bool downward_pass(Ctx* c, cudaStream_t s) {
     if (cnt <= 0) continue;
     COUNT_LAUNCH();
     const unsigned gl = (unsigned)std::min<int64_t>((cnt + kTwigs - 1) / kTwigs, 148 * 16);
-    k_adj_down<<<gl, kDownThreads, 0, s>>>(L, L, D, nullptr, c->d_status);
+    k_adj_down<<<gl, kDownThreads, 0, s>>>(L, L, D, GridBarrier{});
   }
   return true;
 }

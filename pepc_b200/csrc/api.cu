@@ -951,6 +951,13 @@ int pepcg_gather_device(void* ctx, const double* d_in, double* d_out) {
 
 void pepcg_debug_fail_allocations(int64_t after) { g_fail_after.store(after < 0 ? -1 : after); }
 
+int pepcg_debug_barrier_tries(void* ctx, int64_t tries) {
+  Ctx* c = as_ctx(ctx);
+  if (!c) return PEPCG_ERR_BAD_ARG;
+  c->barrier_tries = tries < 0 ? kBarrierTries : (unsigned)std::min<int64_t>(tries, kBarrierTries);
+  return PEPCG_OK;
+}
+
 int pepcg_sort_keys_device(void* ctx, int64_t n, const int64_t* d_keys, int64_t* d_keys_out,
                            int64_t* d_perm_out) {
   Ctx* c = as_ctx(ctx);

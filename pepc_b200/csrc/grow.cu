@@ -524,8 +524,7 @@ __global__ void k_scan_apply(ScanPair<T> a, int64_t n, const T* __restrict__ bsu
 // three paired scans of 16,411 particles take 16 us instead of 22 (ncu).
 template <class T>
 __global__ void __launch_bounds__(kThreads) k_scan_coop(ScanPair<T> a, int64_t n, T* bsum,
-                                                        unsigned* word, uint32_t* status,
-                                                        SummaryArgs S) {
+                                                        GridBarrier B, SummaryArgs S) {
   __shared__ T sm[32];
   const int64_t base = (int64_t)blockIdx.x * kScanTile;
   const T* in = blockIdx.y ? a.in[1] : a.in[0];
@@ -540,7 +539,7 @@ __global__ void __launch_bounds__(kThreads) k_scan_coop(ScanPair<T> a, int64_t n
   T ex = block_exclusive_scan<T>(s, sm, tot);
   if (gridDim.x > 1) {
     if (threadIdx.x == 0) __stcg(bs + blockIdx.x, tot);
-    if (!grid_barrier(word, gridDim.x * gridDim.y, status)) return;
+    if (!grid_barrier(B, gridDim.x * gridDim.y)) return;
     T pre = 0;
     for (int b = threadIdx.x; b < (int)blockIdx.x; b += blockDim.x) pre += __ldcg(bs + b);
     T t;
@@ -569,16 +568,16 @@ __global__ void k_grow_summary(int64_t n, const int32_t* __restrict__ sstart,
 }
 
 // exclusive scans of one array, or of two arrays of the same length in the
-// same launches (tmp: one block sum per 2048 elements and array).  word, status: a
-// zeroed barrier word and the status word that let small arrays take one launch
+// same launches (tmp: one block sum per 2048 elements and array).  bar: a barrier with
+// a zeroed word lets small arrays take one launch
 template <class T>
 void exclusive_scan2(const T* in0, T* out0, const T* in1, T* out1, int64_t n, T* tmp,
-                     cudaStream_t s, unsigned* word = nullptr, uint32_t* status = nullptr,
+                     cudaStream_t s, const GridBarrier& bar = GridBarrier{},
                      const SummaryArgs& sum = SummaryArgs{}) {
   const int64_t nb = (n + kScanTile - 1) / kScanTile;
   ScanPair<T> a{{in0, in1}, {out0, out1}};
   const dim3 grid((unsigned)nb, in1 ? 2u : 1u);
-  if (word && nb <= kScanCoopTiles) {
+  if (bar.word && nb <= kScanCoopTiles) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kThreads);
@@ -588,7 +587,7 @@ void exclusive_scan2(const T* in0, T* out0, const T* in1, T* out1, int64_t n, T*
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_scan_coop<T>, a, n, tmp, word, status, sum) == cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, k_scan_coop<T>, a, n, tmp, bar, sum) == cudaSuccess) {
       COUNT_LAUNCH();
       return;
     }
@@ -657,8 +656,7 @@ struct CoopSortArgs {
   uint64_t *k0, *k1;  // input in k0, v0; the passes alternate
   int32_t *v0, *v1;
   uint32_t* hist;  // kMaxDigits per tile
-  unsigned* word;  // grid barrier
-  uint32_t* status;
+  GridBarrier bar;
   int64_t* ko;     // grow keys: the sorted keys, twice
   int64_t* korig;
   unsigned long long* dupcount;
@@ -747,7 +745,7 @@ __device__ __forceinline__ bool coop_pass(const CoopSortArgs& A, int from, int s
   }
   const uint32_t ls = digit_scan<D>(run, wtot);
   if (tid < D) lstart[tid] = ls;
-  if (nb > 1 && !grid_barrier(A.word, ++barriers * nb, A.status)) return false;
+  if (nb > 1 && !grid_barrier(A.bar, ++barriers * nb)) return false;
   uint32_t tot = 0, pre = 0;
   if (tid < D) {
     const uint32_t* col = A.hist + tid;
@@ -780,7 +778,7 @@ __device__ __forceinline__ bool coop_pass(const CoopSortArgs& A, int from, int s
     vout[dst] = sv[i];
   }
   // the output is complete; also, sk, sv and the counts may be written again
-  if (nb > 1) return grid_barrier(A.word, ++barriers * nb, A.status);
+  if (nb > 1) return grid_barrier(A.bar, ++barriers * nb);
   __syncthreads();
   return true;
 }
@@ -929,7 +927,9 @@ __global__ void k_gather(int64_t n, const int32_t* __restrict__ sval,
                          int32_t* __restrict__ perm, const int64_t* __restrict__ key,
                          const int64_t* __restrict__ korig,
                          const unsigned long long* __restrict__ dupcount, int dupcap,
-                         const double* __restrict__ box, int curve) {
+                         const double* __restrict__ box, int curve,
+                         const uint32_t* __restrict__ status) {
+  if (*status & ST_TIMEOUT) return;  // no sorted indices
   const unsigned long long nd = *dupcount;
   const bool fixed = nd > 0 && nd <= (unsigned long long)dupcap;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -984,6 +984,7 @@ __global__ void k_node_counts(int64_t n, const int64_t* __restrict__ key,
                               int8_t* __restrict__ lev, int8_t* __restrict__ lcpn,
                               int32_t* __restrict__ cstart, int32_t* __restrict__ cend,
                               uint32_t* status, int* maxlev, int32_t* __restrict__ lvl) {
+  if (*status & ST_TIMEOUT) return;  // no sorted keys: lcp_keys of any two words may be negative
   __shared__ int h[kMaxLevel + 1];
   __shared__ int bmax;
   if (threadIdx.x <= kMaxLevel) h[threadIdx.x] = 0;
@@ -1526,8 +1527,7 @@ __global__ void __launch_bounds__(kUpThreads) k_upward_level(int level, UpArgs A
 
 // All levels in one cooperative launch, a grid barrier between them; the list
 // entries of a block's first twigs of the next level are read before it.
-__global__ void __launch_bounds__(kUpThreads) k_upward_all(int top, UpArgs A, unsigned* word,
-                                                          uint32_t* status) {
+__global__ void __launch_bounds__(kUpThreads) k_upward_all(int top, UpArgs A, GridBarrier B) {
   __shared__ double s_t[kUpThreads / 8 * kUpRows * kUpRow];
   __shared__ int s_cnt[kMaxLevel + 1], s_base[kMaxLevel + 1];
   double* T = s_t + (threadIdx.x >> 3) * (kUpRows * kUpRow);
@@ -1549,7 +1549,7 @@ __global__ void __launch_bounds__(kUpThreads) k_upward_all(int top, UpArgs A, un
     if (level > 0) {
       h = twig_head(A, s_base[level - 1] + first, first < s_cnt[level - 1]);
       if (gridDim.x > 1) {
-        if (!grid_barrier(word, ++barriers * gridDim.x, status)) return;
+        if (!grid_barrier(B, ++barriers * gridDim.x)) return;
       } else {
         __syncthreads();
       }
@@ -1737,7 +1737,9 @@ void exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, int32_t* tmp
 }
 
 // k_sort_coop for arrays of up to 148 tiles; false: not launched (see lsd_sort).
-// The barrier word must be zero.
+// The barrier word must be zero.  If a barrier gives up, no sorted key or index stands
+// in the output (the alternate buffers of a new context were never written): the
+// kernels that index by them, and count levels by the keys, look at the status first.
 template <bool kGrow>
 static bool coop_sort(Ctx* c, int64_t n, int dupcap, cudaStream_t s) {
   CoopSortArgs A{};
@@ -1745,8 +1747,7 @@ static bool coop_sort(Ctx* c, int64_t n, int dupcap, cudaStream_t s) {
   A.k0 = c->skey.p; A.k1 = c->skey_alt.p;
   A.v0 = c->sval.p; A.v1 = c->sval_alt.p;
   A.hist = c->hist.p;
-  A.word = c->barrier_word(0);
-  A.status = c->d_status;
+  A.bar = c->barrier(0, c->d_status);
   A.ko = c->key.p;
   A.korig = c->orig_key.p;
   A.dupcount = c->d_small;
@@ -1862,7 +1863,7 @@ static void upward_pass(Ctx* c, const UpArgs& U, cudaStream_t s) {
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_upward_all, c->max_level - 1, U, c->barrier_word(1), c->d_tree_status) ==
+    if (cudaLaunchKernelEx(&cfg, k_upward_all, c->max_level - 1, U, c->barrier(1, c->d_tree_status)) ==
         cudaSuccess) {
       COUNT_LAUNCH();
       return;
@@ -1957,7 +1958,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
   // the host needs the node count M (grid sizes, allocations), the box, the level
   // counts and the status: the scan's last block writes them to mapped host memory
   exclusive_scan2<int32_t>(c->cstart.p, c->sstart.p, c->cend.p, c->send.p, n, c->scan_tmp.p, s,
-                           c->barrier_word(4), c->d_status,
+                           c->barrier(4, c->d_status),
                            SummaryArgs{c->d_box, c->d_small, c->d_status, c->lvlcnt, c->d_sum});
   if (!cuda_ok(c, cudaEventRecord(c->sum_ev, s), "grow summary")) return PEPCG_ERR_CUDA;
   cudaEventRecord(c->ev[9], s);
@@ -1967,7 +1968,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
   k_gather<<<grid_for(n), kThreads, 0, s>>>(n, vin, c->packed.p, q_ready ? dq : nullptr, c->x.p,
                                             c->y.p, c->z.p, c->q.p, c->perm.p, c->key.p,
                                             c->orig_key.p, c->d_small, dupcap, c->d_box,
-                                            c->prm.curve);
+                                            c->prm.curve, c->d_status);
   cudaEventRecord(c->ev[2], s);
   if (c->far_field && !lattice_timestep(c, n, c->ev[2])) return PEPCG_ERR_CUDA;
   if (!cuda_ok(c, cudaEventSynchronize(c->sum_ev), "grow (keys/sort)")) return PEPCG_ERR_CUDA;
@@ -2026,16 +2027,16 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
   // twigs by level, then one launch per level, sized by the level's twig
   // count; the deepest twig level is one above the deepest leaf level
   {
-    exclusive_scan2<int32_t>(bt, bt, ba, ba, (int64_t)nlb, c->scan_tmp.p, s, c->barrier_word(5),
-                             c->d_tree_status);
+    exclusive_scan2<int32_t>(bt, bt, ba, ba, (int64_t)nlb, c->scan_tmp.p, s,
+                             c->barrier(5, c->d_tree_status));
     COUNT_LAUNCH();
     int32_t* cc = c->tcounts.p;
     int32_t* tcn = c->tcounts.p + ntw;
     k_level_scatter<<<gM, kThreads, 0, s>>>(M, c->meta.p, bt, ba, (int)gM, c->twiglist.p,
                                             c->nc4.p, c->drec.p, c->lvlpos.p, c->child8.p,
                                             c->nchild.p, c->tinfo.p, cc, tcn);
-    exclusive_scan2<int32_t>(cc, cc, tcn, tcn, ntw, c->scan_tmp.p, s, c->barrier_word(6),
-                             c->d_tree_status);
+    exclusive_scan2<int32_t>(cc, cc, tcn, tcn, ntw, c->scan_tmp.p, s,
+                             c->barrier(6, c->d_tree_status));
     UpArgs U{c->lvlcnt, c->twiglist.p, c->tinfo.p, cc, tcn, c->nleaves.p, c->drec.p,
              c->dmom.p, c->nc4.p, c->mom.p, reinterpret_cast<float4*>(c->mom32.p)};
     upward_pass(c, U, s);

@@ -93,22 +93,34 @@ __device__ __forceinline__ void st256f(void* p, float4 a, float4 b) {
 // word that was zero at the launch.  Writes before it are visible after it to
 // plain loads (never ld.global.nc) of every block: thread 0's fences order the block's
 // accesses on both sides, as cooperative_groups' grid.sync does.  The wait is
-// bounded (seconds): if it runs out the status word gets ST_TIMEOUT and every
-// thread of the block sees false and returns.
+// bounded (seconds): a block whose tries run out closes the word, unless the
+// barrier completes first, and no block passes a closed one: the status word gets
+// ST_TIMEOUT, every thread of every block sees false and returns.  So what a kernel
+// writes after its last barrier is written by all its blocks or by none.  No tries at
+// all (tests): the first block to arrive closes the word.
 constexpr unsigned kBarrierTries = 1u << 22;
-__device__ __forceinline__ bool grid_barrier(unsigned* word, unsigned target, uint32_t* status) {
+constexpr unsigned kBarrierClosed = 1u << 31;
+struct GridBarrier {
+  unsigned* word;
+  uint32_t* status;
+  unsigned tries;
+};
+__device__ __forceinline__ bool grid_barrier(const GridBarrier& B, unsigned target) {
   __syncthreads();
   int late = 0;
   if (threadIdx.x == 0) {
     __threadfence();
-    atomicAdd(word, 1u);
-    unsigned seen = 0, tries = 0;
-    do {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(word) : "memory");
-    } while (seen < target && ++tries < kBarrierTries);
-    if (seen < target) {
+    unsigned seen = B.tries ? atomicAdd(B.word, 1u) + 1u
+                            : atomicOr(B.word, kBarrierClosed) | kBarrierClosed;
+    for (unsigned t = 0; seen < target && t < B.tries; ++t)
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(B.word) : "memory");
+    while (seen < target) {  // a failed exchange is another block's arrival
+      const unsigned old = atomicCAS(B.word, seen, seen | kBarrierClosed);
+      seen = old == seen ? seen | kBarrierClosed : old;
+    }
+    if (seen & kBarrierClosed) {
       late = 1;
-      atomicOr(status, ST_TIMEOUT);
+      atomicOr(B.status, ST_TIMEOUT);
     }
     __threadfence();
   }
@@ -285,6 +297,8 @@ struct Ctx {
   unsigned long long* item_queue() { return d_small + 10; }
   // counting words of the cooperative kernels' barriers, zeroed before each launch
   unsigned int* barrier_word(int k) { return reinterpret_cast<unsigned int*>(d_small + 16) + k; }
+  unsigned barrier_tries = kBarrierTries;  // tests lower it (pepcg_debug_barrier_tries)
+  GridBarrier barrier(int k, uint32_t* status) { return GridBarrier{barrier_word(k), status, barrier_tries}; }
 };
 
 // The lanes of one pack of the packed per-tile walks: pack b holds the whole

@@ -219,7 +219,7 @@ __device__ void tie_insertion_sort(const TieArgs& a, int r0, int r1) {
 }
 
 __global__ void __launch_bounds__(kTieThreads, 1) k_tie_order(TieArgs a) {
-  if (*a.ndup == 0) return;
+  if (*a.ndup == 0 || (*a.status & ST_TIMEOUT)) return;  // after a sort that gave up sval is no permutation
   extern __shared__ __align__(16) int tsm[];
   TieShared sh;
   sh.cnt = tsm;

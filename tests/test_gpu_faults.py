@@ -4,7 +4,12 @@ Device allocations fail on demand through pepcg_debug_fail_allocations (a
 host-side injection: the allocation call is answered with an error before it
 reaches the device).  A grow or traverse that meets the failure must return
 PEPCG_ERR_OOM with a message, leave no tree behind, and the same context must
-then work again and give the results of a fresh context."""
+then work again and give the results of a fresh context.
+
+The grid barriers of the cooperative kernels give up at once with no tries
+(pepcg_debug_barrier_tries): the call that needed one must return
+PEPCG_ERR_TIMEOUT, read nothing that the kernel did not write, and the context
+must work again."""
 import numpy as np
 import pytest
 
@@ -58,4 +63,53 @@ def test_traverse_allocation_failure_keeps_the_tree(no_injection):
     P.lib().pepcg_debug_fail_allocations(-1)
     r = tc.pepc_traverse_tree(g.x, g.y, g.z, keys=g.key)
     assert np.all(np.isfinite(r["pot"])) and np.all(r["work"] > 0)
+    tc.close()
+
+
+def same_results(tc, x, y, z, q):
+    """tc grows and walks as a fresh context does."""
+    ref = P.TreeCode(theta2=0.25, eps2=1e-4)
+    out = []
+    for t in (ref, tc):
+        g = t.pepc_grow_tree(x, y, z, q)
+        r = t.pepc_traverse_tree(g.x, g.y, g.z, keys=g.key)
+        out.append([g.perm, g.key] + [r[k] for k in ("ex", "ey", "ez", "pot", "work")])
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+    ref.close()
+
+
+# one tile of the sort is 1,024 keys up to 32,768, 2,048 up to 131,072, then 4,096; up to
+# 1,024 keys it has no barrier
+@pytest.mark.parametrize("used", [False, True])
+@pytest.mark.parametrize("n", [1025, 16411, 100003, 600001])
+def test_sort_gives_up_then_recovery(gpu, n, used):
+    x, y, z, q = cube(n, 83, charges="normal")
+    for a in (x, y, z):  # some equal keys
+        a[1:100:2] = a[0:99:2]
+    tc = P.TreeCode(theta2=0.25, eps2=1e-4)
+    if used:  # else every buffer of the context is fresh memory
+        tc.pepc_grow_tree(*cube(n + 1000, 84, charges="normal"))
+    P.lib().pepcg_debug_barrier_tries(tc._h, 0)
+    with pytest.raises(P.PepcgError) as e:
+        tc.pepc_grow_tree(x, y, z, q)
+    assert e.value.code == P.PEPCG_ERR_TIMEOUT
+    with pytest.raises(P.PepcgError) as e:
+        tc.pepc_traverse_tree(x[:10], y[:10], z[:10])
+    assert e.value.code == P.PEPCG_ERR_NO_TREE
+    P.lib().pepcg_debug_barrier_tries(tc._h, -1)
+    same_results(tc, x, y, z, q)
+    tc.close()
+
+
+@pytest.mark.parametrize("n", [1025, 30011])
+def test_key_sort_gives_up_then_recovery(gpu, n):
+    keys = np.random.default_rng(85).integers(0, n // 2, n)  # with equal keys
+    tc = P.TreeCode()
+    P.lib().pepcg_debug_barrier_tries(tc._h, 0)
+    with pytest.raises(P.PepcgError) as e:
+        tc.sort_keys(keys)
+    assert e.value.code == P.PEPCG_ERR_TIMEOUT
+    P.lib().pepcg_debug_barrier_tries(tc._h, -1)
+    ko, po = tc.sort_keys(keys)
+    assert np.array_equal(ko, np.sort(keys)) and np.array_equal(keys[po], ko)
     tc.close()
