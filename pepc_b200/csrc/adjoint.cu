@@ -626,9 +626,11 @@ __global__ void k_reset_adj(unsigned int* q, unsigned long long* items) {
   *items = 0;
 }
 
-// *flag (mapped host memory, zero before the launch) = 1 if any value is not zero
+// *flag (mapped host memory, zero before the launch) = 1 if any value is not zero;
+// *seen (mapped, zero) = *status if that is set (a write to the host costs the wait 2 us)
 __global__ void k_any_nonzero(int64_t n, const double* a, const double* b, const double* c,
-                              uint32_t* flag) {
+                              uint32_t* flag, const uint32_t* status, uint32_t* seen) {
+  if (blockIdx.x == 0 && threadIdx.x == 0 && *status) *seen = *status;
   bool any = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
@@ -727,9 +729,10 @@ int adjoint_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const
   if (!cuda_ok(c, cudaMemsetAsync(c->adj.p, 0, sizeof(double) * kNA * M, s), "adjoint"))
     return PEPCG_ERR_CUDA;
   // is dL/dE zero everywhere?  (then the Hessian terms are skipped)
-  c->h_sum->with_e = 0;  // every earlier call that wrote it has been waited for
+  c->h_sum->with_e = c->h_sum->tree_status = 0;  // every earlier call that wrote them has been waited for
   COUNT_LAUNCH();
-  k_any_nonzero<<<148, 256, 0, s>>>(nt, gex, gey, gez, &c->d_sum->with_e);
+  k_any_nonzero<<<148, 256, 0, s>>>(nt, gex, gey, gez, &c->d_sum->with_e, c->d_tree_status,
+                                   &c->d_sum->tree_status);
   AdjArgs A;
   A.nt = nt;
   A.tx = tx; A.ty = ty; A.tz = tz;
@@ -799,6 +802,8 @@ int adjoint_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const
   }
   if (!cuda_ok(c, cudaStreamSynchronize(s), "flag")) return PEPCG_ERR_CUDA;
   const uint32_t h_flag = *const_cast<volatile uint32_t*>(&c->h_sum->with_e);
+  if (const uint32_t st = *const_cast<volatile uint32_t*>(&c->h_sum->tree_status))
+    return status_to_code(c, st);
   COUNT_LAUNCH();
   k_reset_adj<<<1, 1, 0, s>>>(A.queue, A.item_queue);
   const int blocks = 148 * 8;

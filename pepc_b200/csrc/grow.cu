@@ -929,8 +929,8 @@ __global__ void k_gather(int64_t n, const int32_t* __restrict__ sval,
                          const unsigned long long* __restrict__ dupcount, int dupcap,
                          const double* __restrict__ box, int curve,
                          const uint32_t* __restrict__ status) {
-  if (*status & ST_TIMEOUT) return;  // no sorted indices
   const unsigned long long nd = *dupcount;
+  if (*status & ST_TIMEOUT) return;  // no sorted indices
   const bool fixed = nd > 0 && nd <= (unsigned long long)dupcap;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -984,12 +984,13 @@ __global__ void k_node_counts(int64_t n, const int64_t* __restrict__ key,
                               int8_t* __restrict__ lev, int8_t* __restrict__ lcpn,
                               int32_t* __restrict__ cstart, int32_t* __restrict__ cend,
                               uint32_t* status, int* maxlev, int32_t* __restrict__ lvl) {
-  if (*status & ST_TIMEOUT) return;  // no sorted keys: lcp_keys of any two words may be negative
   __shared__ int h[kMaxLevel + 1];
   __shared__ int bmax;
+  const uint32_t st = *status;
   if (threadIdx.x <= kMaxLevel) h[threadIdx.x] = 0;
   if (threadIdx.x == 0) bmax = 0;
   __syncthreads();
+  if (st & ST_TIMEOUT) return;  // no sorted keys: lcp_keys of any two words may be negative
   int mymax = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -1242,13 +1243,15 @@ __global__ void __launch_bounds__(256) k_level_scatter(int64_t M, const int2* __
                                                        const int32_t* __restrict__ nchild,
                                                        int2* __restrict__ tinfo,
                                                        int32_t* __restrict__ ccnt,
-                                                       int32_t* __restrict__ tcnt) {
+                                                       int32_t* __restrict__ tcnt,
+                                                       const uint32_t* __restrict__ status) {
   __shared__ int wt[256 / 32][kMaxLevel + 1], wa[256 / 32][kMaxLevel + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x < (256 / 32) * (kMaxLevel + 1)) {
     (&wt[0][0])[threadIdx.x] = 0;
     (&wa[0][0])[threadIdx.x] = 0;
   }
+  const uint32_t st = *status;
   const int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int L = -1, end = 0;
   bool leaf = false;
@@ -1259,6 +1262,7 @@ __global__ void __launch_bounds__(256) k_level_scatter(int64_t M, const int2* __
     end = mu.x;
   }
   __syncthreads();
+  if (st & ST_TIMEOUT) return;  // no offsets
   const int rt = block_rank(leaf ? -1 : L, warp, lane, wt);
   const int ra = block_rank(L, warp, lane, wa);
   __syncthreads();
@@ -1329,6 +1333,7 @@ struct UpArgs {
   double4* nc4;
   double* mom;
   float4* mom32;
+  const uint32_t* status;  // of the scans before it: no lists after a barrier gave up
 };
 
 // ld256 that stays where it is written: for records that the running kernel wrote
@@ -1517,8 +1522,10 @@ __device__ __forceinline__ void upward_twig(const UpArgs& A, int level, const Tw
 __global__ void __launch_bounds__(kUpThreads) k_upward_level(int level, UpArgs A) {
   __shared__ double s_t[kUpThreads / 8 * kUpRows * kUpRow];
   double* T = s_t + (threadIdx.x >> 3) * (kUpRows * kUpRow);
+  const uint32_t st = *A.status;
   const int cnt = A.lvl[level];
   const int base = level_base(A.lvl, level);
+  if (st & ST_TIMEOUT) return;
   for (int i0 = blockIdx.x * (kUpThreads / 8); i0 < cnt; i0 += gridDim.x * (kUpThreads / 8)) {
     const int i = i0 + (threadIdx.x >> 3);
     upward_twig(A, level, twig_head(A, base + i, i < cnt), T);
@@ -1531,11 +1538,13 @@ __global__ void __launch_bounds__(kUpThreads) k_upward_all(int top, UpArgs A, Gr
   __shared__ double s_t[kUpThreads / 8 * kUpRows * kUpRow];
   __shared__ int s_cnt[kMaxLevel + 1], s_base[kMaxLevel + 1];
   double* T = s_t + (threadIdx.x >> 3) * (kUpRows * kUpRow);
+  const uint32_t st = *A.status;
   if (threadIdx.x <= kMaxLevel) {
     s_cnt[threadIdx.x] = A.lvl[threadIdx.x];
     s_base[threadIdx.x] = level_base(A.lvl, threadIdx.x);
   }
   __syncthreads();
+  if (st & ST_TIMEOUT) return;
   const int step = gridDim.x * (kUpThreads / 8);
   const int first = blockIdx.x * (kUpThreads / 8) + (threadIdx.x >> 3);
   unsigned barriers = 0;
@@ -1573,8 +1582,10 @@ __global__ void __launch_bounds__(kUpThreads) k_upward_wide(int level, UpArgs A)
   double4* __restrict__ nc4 = A.nc4;
   double* __restrict__ mom = A.mom;
   float4* __restrict__ mom32 = A.mom32;
+  const uint32_t st = *A.status;
   const int cnt = A.lvl[level];
   const int base = level_base(A.lvl, level);
+  if (st & ST_TIMEOUT) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
     const int P = base + i;
     const int64_t u = twiglist[P];
@@ -2034,11 +2045,11 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
     int32_t* tcn = c->tcounts.p + ntw;
     k_level_scatter<<<gM, kThreads, 0, s>>>(M, c->meta.p, bt, ba, (int)gM, c->twiglist.p,
                                             c->nc4.p, c->drec.p, c->lvlpos.p, c->child8.p,
-                                            c->nchild.p, c->tinfo.p, cc, tcn);
+                                            c->nchild.p, c->tinfo.p, cc, tcn, c->d_tree_status);
     exclusive_scan2<int32_t>(cc, cc, tcn, tcn, ntw, c->scan_tmp.p, s,
                              c->barrier(6, c->d_tree_status));
     UpArgs U{c->lvlcnt, c->twiglist.p, c->tinfo.p, cc, tcn, c->nleaves.p, c->drec.p,
-             c->dmom.p, c->nc4.p, c->mom.p, reinterpret_cast<float4*>(c->mom32.p)};
+             c->dmom.p, c->nc4.p, c->mom.p, reinterpret_cast<float4*>(c->mom32.p), c->d_tree_status};
     upward_pass(c, U, s);
   }
   cudaEventRecord(c->ev[4], s);
@@ -2182,6 +2193,7 @@ int export_tree(Ctx* c, int64_t* key, int32_t* level, int64_t* leaves, int64_t* 
                                             c->parent.p, c->nkey.p, c->nc4.p, c->mom.p,
                                             dk, dlev, dl, dd, dp, df, dn, dm, c->first_part.p, c->n);
   bool ok = true;
+  uint32_t st = 0;
   auto cp = [&](void* h, const void* dv, size_t b) {
     if (h) ok = ok && cuda_ok(c, cudaMemcpyAsync(h, dv, b, cudaMemcpyDeviceToHost, s), "export");
   };
@@ -2193,9 +2205,10 @@ int export_tree(Ctx* c, int64_t* key, int32_t* level, int64_t* leaves, int64_t* 
   cp(first_child, df, 8 * M);
   cp(next_sibling, dn, 8 * M);
   cp(mom15, dm, 8 * 15 * M);
+  cp(&st, c->d_tree_status, sizeof(st));
   cudaFreeAsync(d, s);
   if (!ok || !cuda_ok(c, cudaStreamSynchronize(s), "export")) return PEPCG_ERR_CUDA;
-  return PEPCG_OK;
+  return status_to_code(c, st);
 }
 
 }  // namespace pepcg

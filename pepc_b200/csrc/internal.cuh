@@ -208,7 +208,9 @@ struct Ctx {
   // small device state: box (9), boxlength2 (21), status word, dup count ...
   double* d_box = nullptr;    // [0..8] box, [9..29] boxlength2
   // status words: of the running call, and (d_tree_status) of the tree's later kernels
-  // (upward pass, adjoint), which nothing waits for: read with the next walk's status
+  // (level lists and upward pass), which the grow does not wait for.  While it is set,
+  // the level-ordered records hold no links: the walks by them do nothing and report
+  // it, the adjoint looks before it launches, the export with its copies.
   uint32_t* d_status = nullptr;
   // [0] dup count, [1] nnodes, [2] tile count, ...; [8], [9] walk bucket queues (one per
   // walk stream), [10] adjoint item queue, [11] equal pairs, [12] .. [15] interaction
@@ -239,6 +241,7 @@ struct Ctx {
     uint32_t walk_status;           // status words, buckets left to the warp walks
     int32_t nover;
     uint32_t with_e;                // the adjoint's dL/dE is not zero everywhere
+    uint32_t tree_status;           // d_tree_status as the adjoint found it
   };
   GrowSummary* h_sum = nullptr;  // host address
   GrowSummary* d_sum = nullptr;  // its device address

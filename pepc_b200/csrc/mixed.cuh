@@ -47,6 +47,7 @@ struct MixArgs {
   const int32_t* tflag;  // per target: length of the tile starting there, else 0
   const int32_t* pstart;  // packed per-tile walk: first target of each pack, then nt
   const int32_t* npacks;  // the number of packs (device)
+  const uint32_t* tree_status;  // set: drec was not built
 };
 
 // 1/sqrt(x) by the PTX instruction rsqrt.approx.ftz.f32 (relative error below

@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(32 * W, walk_block_resident<W, kStrict>())
   for (int i = tid; i < 3 * A.nbox; i += kThreads) s_vb[i] = A.vbox[i];
   int* stack = gstack + (int64_t)blockIdx.x * W * kStackCap;
   const int part = nparts > 1 ? (int)(blockIdx.x % nparts) : 0;
-  const int64_t nbuckets = (A.nt + 63) / 64;
+  const int64_t nbuckets = *A.tree_status & ST_TIMEOUT ? 0 : (A.nt + 63) / 64;
   const BlockTree B{A.drec, A.mom32, A.macb, A.theta2, A.theta2d};
   unsigned long long c_leaf = 0, c_twig = 0, c_mac = 0;
   for (bool first = true;; first = false) {

@@ -332,6 +332,7 @@ __global__ void __launch_bounds__(kMixThreads, kStrict ? 4 : 5)
     if constexpr (kStrict) s_bl2d[i] = A.bl2[i];
   }
   for (int i = threadIdx.x; i < 3 * A.nbox; i += blockDim.x) s_vb[i] = A.vbox[i];
+  const uint32_t st = *A.tree_status;
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(kMixThreads, kStrict ? 4 : 5)
   TwigRec* stw = s_tw[w];
   StagedLeaf* stl = s_lf[w];
   const float theta2 = A.theta2;
-  const int64_t nbuckets = (A.nt + 63) / 64;
+  const int64_t nbuckets = st & ST_TIMEOUT ? 0 : (A.nt + 63) / 64;
   unsigned long long c_leaf = 0, c_twig = 0, c_mac = 0;
   for (;;) {
     unsigned b = 0;
@@ -1069,6 +1070,7 @@ int launch_walk_mixed(Ctx* c, int64_t nt, const double* tx, const double* ty, co
   A.tflag = tflag;
   A.pstart = pstart;
   A.npacks = npacks;
+  A.tree_status = c->d_tree_status;
   BlockShape sh;
   const bool group64 = !per_target && !tflag && tiles == nullptr && c->group_size() == 64;
   const bool strict = c->prm.precision == PEPCG_PRECISION_MIXED_STRICT;

@@ -72,6 +72,7 @@ struct WalkArgs {
   // what k_walk_list64 left to k_walk_target64 / k_walk_tilepack64 (kOnly): [0] their
   // number, then targets (count << 20 | first) or packs
   int32_t* over;
+  const uint32_t* tree_status;  // set: drec was not built
 };
 
 // any(abs(delta) >= spatial_interaction_cutoff) (module_tree_walk_pthreads.f90:
@@ -489,7 +490,8 @@ __global__ void __launch_bounds__(kListThreads, 2) k_walk_list64(WalkArgs A) {
   const unsigned lt = (1u << lane) - 1u;
   for (int i = tid; i <= kMaxLevel; i += kListThreads) S.bl2[i] = A.bl2[i];
   uint2* stack = A.lstack + (int64_t)blockIdx.x * kListStack;
-  const int64_t nbk = kTile ? (int64_t)*A.npacks : (A.nt + A.lper - 1) / A.lper;
+  const int64_t nbk = *A.tree_status & ST_TIMEOUT ? 0
+                      : kTile ? (int64_t)*A.npacks : (A.nt + A.lper - 1) / A.lper;
   const double vx = A.vbox[0], vy = A.vbox[1], vz = A.vbox[2];
   unsigned long long c_leaf = 0, c_twig = 0, c_mac = 0;
   int64_t b = 0, first = 0;  // bucket, and its targets [first, first + left) to do (per target)
@@ -1113,6 +1115,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
         !ensure(c, c->over, 1 + (packed ? nbk : (int64_t)nt), "walk lists"))
       return PEPCG_ERR_OOM;
     A.drec = c->drec.p;
+    A.tree_status = c->d_tree_status;
     A.rpo2fpo = c->rpo2fpo.p;
     A.fpo2rpo = c->fpo2rpo.p;
     A.lstack = reinterpret_cast<uint2*>(c->wstack.p);

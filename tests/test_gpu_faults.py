@@ -113,3 +113,47 @@ def test_key_sort_gives_up_then_recovery(gpu, n):
     ko, po = tc.sort_keys(keys)
     assert np.array_equal(ko, np.sort(keys)) and np.array_equal(keys[po], ko)
     tc.close()
+
+
+WALKS = [(P.PRECISION_PLAIN, P.WALK_PER_TARGET), (P.PRECISION_PLAIN, P.WALK_PER_TILE),
+         (P.PRECISION_PLAIN, P.WALK_GROUP), (P.PRECISION_MIXED, P.WALK_PER_TARGET),
+         (P.PRECISION_MIXED, P.WALK_PER_TILE), (P.PRECISION_MIXED, P.WALK_GROUP),
+         (P.PRECISION_MIXED_STRICT, P.WALK_GROUP)]
+
+
+@pytest.mark.parametrize("precision,walk", WALKS)
+def test_upward_pass_gives_up_and_every_reader_says_so(gpu, precision, walk):
+    # up to 1,024 keys the sort has no barrier and the scans (one tile) have none, the
+    # upward pass has: the grow returns before it
+    x, y, z, q = cube(1000, 86, charges="normal")
+    kw = dict(theta2=0.25, eps2=1e-4, precision=precision, walk=walk)
+    tc, ref = P.TreeCode(**kw), P.TreeCode(**kw)
+    P.lib().pepcg_debug_barrier_tries(tc._h, 0)
+    g = tc.pepc_grow_tree(x, y, z, q)
+    zero, one = np.zeros(1000), np.ones(1000)
+    for call in (lambda: tc.pepc_traverse_tree(g.x, g.y, g.z, keys=g.key),
+                 lambda: tc.traverse_adjoint(g.x, g.y, g.z, [zero] * 3, one, 1000),
+                 tc.tree):
+        with pytest.raises(P.PepcgError) as e:
+            call()
+        assert e.value.code == P.PEPCG_ERR_TIMEOUT
+    P.lib().pepcg_debug_barrier_tries(tc._h, -1)
+    tc.pepc_grow_tree(x, y, z, q)
+    ref.pepc_grow_tree(x, y, z, q)
+    a, b = [t.pepc_traverse_tree(g.x, g.y, g.z, keys=g.key) for t in (tc, ref)]
+    assert all(np.array_equal(a[k], b[k]) for k in ("ex", "ey", "ez", "pot", "work"))
+    tc.close()
+    ref.close()
+
+
+def test_group_walk_by_warps_leaves_an_unbuilt_tree_alone(gpu):
+    # more buckets than the walk by blocks takes
+    n, nt = 1000, 9000 * 64 + 1
+    tc = P.TreeCode(theta2=0.25, eps2=1e-4, precision=P.PRECISION_MIXED, walk=P.WALK_GROUP)
+    P.lib().pepcg_debug_barrier_tries(tc._h, 0)
+    tc.pepc_grow_tree(*cube(n, 87, charges="normal"))
+    t = np.random.default_rng(88).random((3, nt))
+    with pytest.raises(P.PepcgError) as e:
+        tc.pepc_traverse_tree(*t)
+    assert e.value.code == P.PEPCG_ERR_TIMEOUT
+    tc.close()
