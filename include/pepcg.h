@@ -204,7 +204,9 @@ int pepcg_traverse_adjoint(void* ctx, int64_t nt, const double* tx, const double
                            const double* tz, const double* dLdEx, const double* dLdEy,
                            const double* dLdEz, const double* dLdphi, double* dLdq, double* dLdx,
                            double* dLdy, double* dLdz);
-/* Same with device arrays. */
+/* Same with device arrays.  The call returns while its kernels run; should one of them
+ * give up (a bounded wait, an incomplete walk), the next grow, traverse, adjoint or
+ * export on the context returns the error in place of its own result. */
 int pepcg_traverse_adjoint_device(void* ctx, int64_t nt, const double* d_tx, const double* d_ty,
                                   const double* d_tz, const double* d_gex, const double* d_gey,
                                   const double* d_gez, const double* d_gphi, double* d_dq,

@@ -603,12 +603,14 @@ __global__ void __launch_bounds__(kDownThreads) k_adj_down(int level, int last, 
   }
 }
 
-// leaves -> particles in the caller's original order
+// leaves -> particles in the caller's original order; *seen (mapped host memory) =
+// *status of the adjoint's kernels, if it is set
 __global__ void k_adj_out(int64_t n, const int32_t* __restrict__ leafnode,
                           const int32_t* __restrict__ lvlpos,
                           const int32_t* __restrict__ perm, const double* __restrict__ q,
                           const double* __restrict__ adj, double* dq, double* dx, double* dy,
-                          double* dz) {
+                          double* dz, const uint32_t* __restrict__ status, uint32_t* seen) {
+  if (blockIdx.x == 0 && threadIdx.x == 0 && *status) *seen = *status;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const double* a = adj + (int64_t)kNA * lvlpos[leafnode[i]];
@@ -621,9 +623,10 @@ __global__ void k_adj_out(int64_t n, const int32_t* __restrict__ leafnode,
   }
 }
 
-__global__ void k_reset_adj(unsigned int* q, unsigned long long* items) {
+__global__ void k_reset_adj(unsigned int* q, unsigned long long* items, uint32_t* status) {
   *q = 0;
   *items = 0;
+  *status = 0;
 }
 
 // *flag (mapped host memory, zero before the launch) = 1 if any value is not zero;
@@ -691,7 +694,7 @@ bool downward_pass(Ctx* c, cudaStream_t s) {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     if (cudaLaunchKernelEx(&cfg, k_adj_down, 0, c->max_level - 1, D,
-                           c->barrier(2, c->d_tree_status)) == cudaSuccess) {
+                           c->barrier(2, c->d_adj_status)) == cudaSuccess) {
       COUNT_LAUNCH();
       return true;
     }
@@ -708,6 +711,16 @@ bool downward_pass(Ctx* c, cudaStream_t s) {
 }
 
 }  // namespace
+
+int take_adjoint_status(Ctx* c) {
+  volatile uint32_t* w = &c->h_sum->adj_status;
+  const uint32_t st = *w;
+  if (!st) return PEPCG_OK;
+  *w = 0;
+  const int rc = status_to_code(c, st);
+  c->err = "the last adjoint's gradients are incomplete: " + c->err;
+  return rc;
+}
 
 int adjoint_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const double* tz,
                    const double* gex, const double* gey, const double* gez, const double* gphi,
@@ -804,8 +817,9 @@ int adjoint_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const
   const uint32_t h_flag = *const_cast<volatile uint32_t*>(&c->h_sum->with_e);
   if (const uint32_t st = *const_cast<volatile uint32_t*>(&c->h_sum->tree_status))
     return status_to_code(c, st);
+  if (const int rc = take_adjoint_status(c)) return rc;  // of the adjoint before this one
   COUNT_LAUNCH();
-  k_reset_adj<<<1, 1, 0, s>>>(A.queue, A.item_queue);
+  k_reset_adj<<<1, 1, 0, s>>>(A.queue, A.item_queue, c->d_adj_status);
   const int blocks = 148 * 8;
   if (mixed64) {
     int rc = launch_adjoint_group64(c, nt, tx, ty, tz, gex, gey, gez, gphi, h_flag != 0, s);
@@ -819,7 +833,7 @@ int adjoint_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const
   if (!downward_pass(c, s)) return PEPCG_ERR_CUDA;
   COUNT_LAUNCH();
   k_adj_out<<<g, 256, 0, s>>>(c->n, c->leafnode.p, c->lvlpos.p, c->perm.p, c->q.p, c->adj.p, dq,
-                              dx, dy, dz);
+                              dx, dy, dz, c->d_adj_status, &c->d_sum->adj_status);
   if (!cuda_ok(c, cudaGetLastError(), "adjoint")) return PEPCG_ERR_CUDA;
   // the periodic far-lattice term's adjoint (FP64, lattice.cu) adds to the walk's
   return c->far_field ? lattice_adjoint(c, nt, tx, ty, tz, gex, gey, gez, gphi, dq, dx, dy, dz)

@@ -6,6 +6,7 @@
 // fallback: without a usable CUDA device every entry point fails with
 // PEPCG_ERR_CUDA.
 
+#include <algorithm>
 #include <cfloat>
 #include <cstdio>
 #include <cstring>
@@ -360,7 +361,9 @@ int pepcg_create(void** out, const pepcg_params* p) {
   c->counters = c->d_small + 12;
   c->d_status = reinterpret_cast<uint32_t*>(c->d_small + 20);
   c->d_tree_status = reinterpret_cast<uint32_t*>(c->d_small + 21);
+  c->d_adj_status = reinterpret_cast<uint32_t*>(c->d_small + 22);
   c->lvlcnt = reinterpret_cast<int32_t*>(c->d_small + 34);
+  std::memset(c->h_sum, 0, sizeof(Ctx::GrowSummary));
   prepare_boxes(c);
   cudaMemcpy(c->d_vbox, c->vbox, 3 * c->nboxes * sizeof(double), cudaMemcpyHostToDevice);
   if (c->far_field) {
@@ -767,7 +770,7 @@ int pepcg_traverse_adjoint(void* ctx, int64_t nt, const double* tx, const double
   for (int k = 0; k < 4; ++k)
     ok = ok && cuda_ok(c, cudaMemcpyAsync(hout[k], o + k * n, n * 8, cudaMemcpyDeviceToHost, s), "D2H");
   ok = ok && cuda_ok(c, cudaStreamSynchronize(s), "adjoint");
-  return ok ? PEPCG_OK : PEPCG_ERR_CUDA;
+  return ok ? take_adjoint_status(c) : PEPCG_ERR_CUDA;
 }
 
 int pepcg_timber_tree(void* ctx) {

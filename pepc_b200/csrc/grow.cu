@@ -1995,6 +1995,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
     cudaStreamSynchronize(s);
     return status_to_code(c, gs.status);
   }
+  if (const int rc = take_adjoint_status(c)) return cudaStreamSynchronize(s), rc;
   const int64_t M = (int64_t)gs.starts_before_last + gs.starts_last;
   // every particle starts at most kMaxLevel + 1 nodes
   if (M < 2 || M > (int64_t)(kMaxLevel + 1) * n || M >= (int64_t)INT32_MAX) {
@@ -2208,7 +2209,8 @@ int export_tree(Ctx* c, int64_t* key, int32_t* level, int64_t* leaves, int64_t* 
   cp(&st, c->d_tree_status, sizeof(st));
   cudaFreeAsync(d, s);
   if (!ok || !cuda_ok(c, cudaStreamSynchronize(s), "export")) return PEPCG_ERR_CUDA;
-  return status_to_code(c, st);
+  if (st) return status_to_code(c, st);
+  return take_adjoint_status(c);
 }
 
 }  // namespace pepcg

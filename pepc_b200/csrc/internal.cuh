@@ -211,15 +211,18 @@ struct Ctx {
   // (level lists and upward pass), which the grow does not wait for.  While it is set,
   // the level-ordered records hold no links: the walks by them do nothing and report
   // it, the adjoint looks before it launches, the export with its copies.
+  // d_adj_status: of the adjoint's kernels; its output kernel passes it on to the host
+  // (h_sum->adj_status), where the next call that waits for the device takes it.
   uint32_t* d_status = nullptr;
   // [0] dup count, [1] nnodes, [2] tile count, ...; [8], [9] walk bucket queues (one per
   // walk stream), [10] adjoint item queue, [11] equal pairs, [12] .. [15] interaction
   // counters, [16] .. [19] grid barriers and block counters (32-bit words), [20]
-  // d_status, [21] d_tree_status, [34] .. lvlcnt: one memset clears all for a grow,
+  // d_status, [21] d_tree_status, [22] d_adj_status, [34] .. lvlcnt: one memset clears all for a grow,
   // one clears [8, 21) for a walk
   unsigned long long* d_small = nullptr;
   unsigned long long* counters = nullptr;
   uint32_t* d_tree_status = nullptr;
+  uint32_t* d_adj_status = nullptr;
   static constexpr int kSmall = 34 + 16;
   double box[9];
   double boxlength2[kMaxLevel + 1];
@@ -242,6 +245,7 @@ struct Ctx {
     int32_t nover;
     uint32_t with_e;                // the adjoint's dL/dE is not zero everywhere
     uint32_t tree_status;           // d_tree_status as the adjoint found it
+    uint32_t adj_status;            // of an adjoint, until a call has reported it
   };
   GrowSummary* h_sum = nullptr;  // host address
   GrowSummary* d_sum = nullptr;  // its device address
@@ -414,6 +418,9 @@ int launch_adjoint_group64(Ctx* c, int64_t nt, const double* tx, const double* t
                            const double* gez, const double* gphi, bool with_e, cudaStream_t s);
 
 // ---- adjoint.cu ----
+// the status that an earlier adjoint left, once (PEPCG_OK: none): its kernels run after
+// the call that launched them has returned.  Called by the host after a wait for the stream
+int take_adjoint_status(Ctx* c);
 int adjoint_device(Ctx* c, int64_t nt, const double* tx, const double* ty, const double* tz,
                    const double* gex, const double* gey, const double* gez, const double* gphi,
                    double* dq, double* dx, double* dy, double* dz);

@@ -1130,7 +1130,7 @@ int launch_adjoint_group64(Ctx* c, int64_t nt, const double* tx, const double* t
   A.npart = c->n;
   A.adj = c->adj.p;
   A.counters = c->counters;
-  A.status = c->d_status;
+  A.status = c->d_adj_status;
   A.queue = c->walk_queue();
   const int gblocks = 148 * 4;
   const size_t per = (size_t)gblocks * kWW * kStackCap;

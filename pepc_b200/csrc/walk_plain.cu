@@ -1225,7 +1225,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   if (cudaEventElapsedTime(&ms, c->ev[5], c->ev[6]) == cudaSuccess) c->st.t_walk_ms = ms;
   if (cudaEventElapsedTime(&ms, c->ev[6], c->ev[7]) == cudaSuccess) c->st.t_lattice_ms = ms;
   if (st) return status_to_code(c, st);
-  return PEPCG_OK;
+  return take_adjoint_status(c);
 }
 
 }  // namespace pepcg

@@ -157,3 +157,49 @@ def test_group_walk_by_warps_leaves_an_unbuilt_tree_alone(gpu):
         tc.pepc_traverse_tree(*t)
     assert e.value.code == P.PEPCG_ERR_TIMEOUT
     tc.close()
+
+
+@pytest.mark.parametrize("precision,walk", WALKS)
+def test_downward_pass_gives_up_in_the_host_adjoint(gpu, precision, walk):
+    n = 3000
+    x, y, z, q = cube(n, 89, charges="normal")
+    tc = P.TreeCode(theta2=0.25, eps2=1e-4, precision=precision, walk=walk)
+    g = tc.pepc_grow_tree(x, y, z, q)
+    args = (g.x, g.y, g.z, [np.zeros(n)] * 3, np.ones(n), n)
+    good = tc.traverse_adjoint(*args)
+    P.lib().pepcg_debug_barrier_tries(tc._h, 0)
+    with pytest.raises(P.PepcgError) as e:
+        tc.traverse_adjoint(*args)
+    assert e.value.code == P.PEPCG_ERR_TIMEOUT and "adjoint" in str(e.value)
+    P.lib().pepcg_debug_barrier_tries(tc._h, -1)
+    again = tc.traverse_adjoint(*args)
+    # FP64 atomics: each sum's some 1e4 terms in another order, 1e4 * 2^-53 of terms that
+    # may cancel to a thousandth
+    for k in good:
+        assert np.abs(again[k] - good[k]).max() <= 1e-9 * np.abs(good[k]).max(), k
+    tc.close()
+
+
+@pytest.mark.parametrize("after", ["grow", "traverse", "adjoint", "export"])
+def test_next_call_reports_a_device_adjoint_that_gave_up(gpu, after):
+    import torch
+    n = 3000
+    p = [torch.from_numpy(v).cuda() for v in cube(n, 90, charges="normal")]
+    tc = P.TreeCode(theta2=0.25, eps2=1e-4, precision=P.PRECISION_MIXED, walk=P.WALK_GROUP)
+    tc.set_stream(torch.cuda.current_stream().cuda_stream)
+    tc.grow_tree_device(*p)
+    f = torch.zeros((9, n), dtype=torch.float64, device="cuda")
+    calls = dict(grow=lambda: tc.grow_tree_device(*p),
+                 traverse=lambda: tc.traverse_self_device(*f[:5]),
+                 adjoint=lambda: tc.traverse_adjoint_device(*p[:3], [f[5]] * 3, torch.ones_like(f[5]),
+                                                            *f[:4]),
+                 export=tc.tree)
+    P.lib().pepcg_debug_barrier_tries(tc._h, 0)
+    calls["adjoint"]()  # returns while its kernels run
+    P.lib().pepcg_debug_barrier_tries(tc._h, -1)
+    with pytest.raises(P.PepcgError) as e:
+        calls[after]()
+    assert e.value.code == P.PEPCG_ERR_TIMEOUT and "adjoint" in str(e.value)
+    for k in ("grow", "traverse", "adjoint", "export", "grow"):  # reported once
+        calls[k]()
+    tc.close()
