@@ -299,6 +299,15 @@ void pepcg_debug_fail_allocations(int64_t after);
  */
 int pepcg_debug_barrier_tries(void* ctx, int64_t tries);
 
+/*
+ * pepcg_debug_refuse -- for tests: what this context treats as refused by the
+ * driver, a sum of
+ *   1  the creation of the second walk stream of the host-array calls (they
+ *      return PEPCG_ERR_CUDA; a later call tries again).
+ * 0 (the default) refuses nothing.
+ */
+int pepcg_debug_refuse(void* ctx, int32_t what);
+
 /* replaces pepc_timber_tree (module_pepc.f90:538 -> module_libpepc_main.f90:129-148) */
 int pepcg_timber_tree(void* ctx);
 int pepcg_stats_get(void* ctx, pepcg_stats* s);

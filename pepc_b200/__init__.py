@@ -124,6 +124,7 @@ EXPORTS = [
     "pepcg_traverse_range_device", "pepcg_restore_device",
     "pepcg_sort_keys", "pepcg_sort_keys_device", "pepcg_lattice_force",
     "pepcg_debug_fail_allocations", "pepcg_debug_barrier_tries",
+    "pepcg_debug_refuse",
 ]
 
 _LIB = None
@@ -168,6 +169,7 @@ def lib():
     L.pepcg_debug_fail_allocations.argtypes = [C.c_int64]
     L.pepcg_debug_fail_allocations.restype = None
     L.pepcg_debug_barrier_tries.argtypes = [VP, C.c_int64]
+    L.pepcg_debug_refuse.argtypes = [VP, C.c_int32]
     L.pepcg_kernel_launches.argtypes = []
     L.pepcg_kernel_launches.restype = C.c_longlong
     L.pepcg_stats_get.argtypes = [VP, C.POINTER(Stats)]

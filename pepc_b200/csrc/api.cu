@@ -314,6 +314,25 @@ const char* pepcg_last_error(const void* ctx) {
   return static_cast<const Ctx*>(ctx)->err.c_str();
 }
 
+static void drop_copy_streams(Ctx* c) {
+  auto drop = [](cudaEvent_t& e) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  };
+  for (int i = 0; i < Ctx::kMaxChunks; ++i) {
+    drop(c->ready[i]);
+    drop(c->done[i]);
+  }
+  drop(c->fork);
+  drop(c->join);
+  for (cudaStream_t* t : {&c->h2d, &c->d2h, &c->walk2})
+    if (*t) {
+      cudaStreamSynchronize(*t);
+      cudaStreamDestroy(*t);
+      *t = nullptr;
+    }
+}
+
 int pepcg_create(void** out, const pepcg_params* p) {
   if (!out || !p) {
     g_static_err = "pepcg_create: null argument";
@@ -409,17 +428,12 @@ int pepcg_destroy(void* ctx) {
   if (c->h_sum) cudaFreeHost(c->h_sum);
   if (c->sum_ev) cudaEventDestroy(c->sum_ev);
   if (c->keys_ev) cudaEventDestroy(c->keys_ev);
-  for (int i = 0; i < Ctx::kMaxChunks; ++i) {
-    if (c->ready[i]) cudaEventDestroy(c->ready[i]);
-    if (c->done[i]) cudaEventDestroy(c->done[i]);
+  drop_copy_streams(c);
+  if (c->lat_ev) cudaEventDestroy(c->lat_ev);
+  if (c->lat_stream) {
+    cudaStreamSynchronize(c->lat_stream);
+    cudaStreamDestroy(c->lat_stream);
   }
-  for (cudaEvent_t e : {c->fork, c->join, c->lat_ev})
-    if (e) cudaEventDestroy(e);
-  for (cudaStream_t t : {c->h2d, c->d2h, c->walk2, c->lat_stream})
-    if (t) {
-      cudaStreamSynchronize(t);
-      cudaStreamDestroy(t);
-    }
   if (c->stream && c->own_stream) cudaStreamDestroy(c->stream);
   delete c;
   return PEPCG_OK;
@@ -446,17 +460,20 @@ int pepcg_set_params(void* ctx, const pepcg_params* p) {
 }
 
 // The copy streams and chunk events of the host-array entry points, created on
-// first use.
+// first use: all of them, or none (the next call tries again).
 static bool copy_streams(Ctx* c) {
   if (c->h2d) return true;
   bool ok = cuda_ok(c, cudaStreamCreateWithFlags(&c->h2d, cudaStreamNonBlocking), "copy stream") &&
             cuda_ok(c, cudaStreamCreateWithFlags(&c->d2h, cudaStreamNonBlocking), "copy stream") &&
-            cuda_ok(c, cudaStreamCreateWithFlags(&c->walk2, cudaStreamNonBlocking), "walk stream") &&
+            cuda_ok(c, c->refuse & kRefuseWalkStream
+                           ? cudaErrorNotSupported
+                           : cudaStreamCreateWithFlags(&c->walk2, cudaStreamNonBlocking), "walk stream") &&
             cuda_ok(c, cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming), "event") &&
             cuda_ok(c, cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming), "event");
   for (int i = 0; ok && i < Ctx::kMaxChunks; ++i)
     ok = cuda_ok(c, cudaEventCreateWithFlags(&c->ready[i], cudaEventDisableTiming), "event") &&
          cuda_ok(c, cudaEventCreateWithFlags(&c->done[i], cudaEventDisableTiming), "event");
+  if (!ok) drop_copy_streams(c);
   return ok;
 }
 
@@ -953,6 +970,13 @@ int pepcg_gather_device(void* ctx, const double* d_in, double* d_out) {
 }
 
 void pepcg_debug_fail_allocations(int64_t after) { g_fail_after.store(after < 0 ? -1 : after); }
+
+int pepcg_debug_refuse(void* ctx, int32_t what) {
+  Ctx* c = as_ctx(ctx);
+  if (!c || what < 0) return PEPCG_ERR_BAD_ARG;
+  c->refuse = (uint32_t)what;
+  return PEPCG_OK;
+}
 
 int pepcg_debug_barrier_tries(void* ctx, int64_t tries) {
   Ctx* c = as_ctx(ctx);

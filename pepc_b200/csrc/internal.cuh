@@ -58,6 +58,9 @@ struct DBuf {
 
 struct Walk;
 
+// what a context treats as refused by the driver (pepcg_debug_refuse, for tests)
+enum : uint32_t { kRefuseWalkStream = 1u << 0 };
+
 // Per-node records are whole 32-byte sectors, so that the upward pass writes
 // no partial sector (a partial sector costs HBM a read-modify-write):
 //   mom  : kMomStride doubles per node, moments [0, 9), abs_charge, bmax, pad
@@ -304,6 +307,7 @@ struct Ctx {
   unsigned long long* item_queue() { return d_small + 10; }
   // counting words of the cooperative kernels' barriers, zeroed before each launch
   unsigned int* barrier_word(int k) { return reinterpret_cast<unsigned int*>(d_small + 16) + k; }
+  uint32_t refuse = 0;                     // kRefuse bits (pepcg_debug_refuse)
   unsigned barrier_tries = kBarrierTries;  // tests lower it (pepcg_debug_barrier_tries)
   GridBarrier barrier(int k, uint32_t* status) { return GridBarrier{barrier_word(k), status, barrier_tries}; }
 };

@@ -1125,7 +1125,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   }
   // chunks alternate between the context stream and walk2, so that each
   // chunk's walk starts while the previous one finishes its last buckets
-  const bool two = nchunks > 1 && c->walk2;
+  const bool two = nchunks > 1;  // a plan comes with walk2 (copy_streams)
   if (two && (!cuda_ok(c, cudaEventRecord(c->fork, s), "fork") ||
               !cuda_ok(c, cudaStreamWaitEvent(c->walk2, c->fork, 0), "fork")))
     return PEPCG_ERR_CUDA;

@@ -203,3 +203,24 @@ def test_next_call_reports_a_device_adjoint_that_gave_up(gpu, after):
     for k in ("grow", "traverse", "adjoint", "export", "grow"):  # reported once
         calls[k]()
     tc.close()
+
+
+@pytest.mark.parametrize("precision", [P.PRECISION_PLAIN, P.PRECISION_MIXED])
+def test_refused_walk_stream_then_recovery(gpu, precision):
+    n = 300001  # host targets in chunks, on two streams
+    x, y, z, q = cube(n, 91, charges="normal")
+    kw = dict(theta2=0.36, eps2=1e-4, precision=precision, walk=P.WALK_GROUP)
+    tc, ref = P.TreeCode(**kw), P.TreeCode(**kw)
+    P.lib().pepcg_debug_refuse(tc._h, 1)
+    for _ in range(2):
+        with pytest.raises(P.PepcgError) as e:
+            tc.pepc_grow_tree(x, y, z, q)
+        assert e.value.code == P.PEPCG_ERR_CUDA and "walk stream" in str(e.value)
+    P.lib().pepcg_debug_refuse(tc._h, 0)
+    out = []
+    for t in (tc, ref):
+        g = t.pepc_grow_tree(x, y, z, q)
+        out.append(t.pepc_traverse_tree(g.x, g.y, g.z, keys=g.key))
+    assert all(np.array_equal(out[0][k], out[1][k]) for k in ("ex", "ey", "ez", "pot", "work"))
+    tc.close()
+    ref.close()
