@@ -303,7 +303,11 @@ int pepcg_debug_barrier_tries(void* ctx, int64_t tries);
  * pepcg_debug_refuse -- for tests: what this context treats as refused by the
  * driver, a sum of
  *   1  the creation of the second walk stream of the host-array calls (they
- *      return PEPCG_ERR_CUDA; a later call tries again).
+ *      return PEPCG_ERR_CUDA; a later call tries again),
+ *   2  cooperative launches (the sort, the scans, the upward pass and the
+ *      adjoint's downward pass then take several launches each),
+ *   4  cluster launches (group walks of few targets then take a warp per
+ *      bucket).
  * 0 (the default) refuses nothing.
  */
 int pepcg_debug_refuse(void* ctx, int32_t what);

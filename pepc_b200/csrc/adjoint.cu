@@ -683,22 +683,10 @@ bool downward_pass(Ctx* c, cudaStream_t s) {
   constexpr int kTwigs = kDownThreads / 8;
   if (widest <= kDownFusedWidest) {
     if (!cuda_ok(c, cudaMemsetAsync(c->barrier_word(2), 0, sizeof(unsigned), s), "adjoint")) return false;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)std::min<int64_t>((widest + kTwigs - 1) / kTwigs,
-                                                   widest > 16384 ? 592 : 296));
-    cfg.blockDim = dim3(kDownThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_adj_down, 0, c->max_level - 1, D,
-                           c->barrier(2, c->d_adj_status)) == cudaSuccess) {
-      COUNT_LAUNCH();
+    const dim3 grid((unsigned)std::min<int64_t>((widest + kTwigs - 1) / kTwigs, widest > 16384 ? 592 : 296));
+    if (launch_cooperative(c, k_adj_down, grid, kDownThreads, 0, s, 0, c->max_level - 1, D,
+                           c->barrier(2, c->d_adj_status)))
       return true;
-    }
-    cudaGetLastError();  // level by level instead
   }
   for (int L = 0; L < c->max_level; ++L) {
     const int64_t cnt = c->lvl_host[L];

@@ -568,31 +568,17 @@ __global__ void k_grow_summary(int64_t n, const int32_t* __restrict__ sstart,
 }
 
 // exclusive scans of one array, or of two arrays of the same length in the
-// same launches (tmp: one block sum per 2048 elements and array).  bar: a barrier with
-// a zeroed word lets small arrays take one launch
+// same launches (tmp: one block sum per 2048 elements and array).  c and bar, a barrier
+// with a zeroed word, let small arrays take one launch
 template <class T>
 void exclusive_scan2(const T* in0, T* out0, const T* in1, T* out1, int64_t n, T* tmp,
-                     cudaStream_t s, const GridBarrier& bar = GridBarrier{},
+                     cudaStream_t s, Ctx* c = nullptr, const GridBarrier& bar = GridBarrier{},
                      const SummaryArgs& sum = SummaryArgs{}) {
   const int64_t nb = (n + kScanTile - 1) / kScanTile;
   ScanPair<T> a{{in0, in1}, {out0, out1}};
   const dim3 grid((unsigned)nb, in1 ? 2u : 1u);
-  if (bar.word && nb <= kScanCoopTiles) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(kThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_scan_coop<T>, a, n, tmp, bar, sum) == cudaSuccess) {
-      COUNT_LAUNCH();
-      return;
-    }
-    cudaGetLastError();  // two launches instead
-  }
+  if (c && nb <= kScanCoopTiles && launch_cooperative(c, k_scan_coop<T>, grid, kThreads, 0, s, a, n, tmp, bar, sum))
+    return;
   COUNT_LAUNCH();
   k_scan_reduce<T><<<grid, kThreads, 0, s>>>(a, n, tmp);
   COUNT_LAUNCH();
@@ -1767,22 +1753,8 @@ static bool coop_sort(Ctx* c, int64_t n, int dupcap, cudaStream_t s) {
   auto go = [&](auto kern, int per, int smem) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return false;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)((n + 512 * per - 1) / (512 * per)));
-    cfg.blockDim = dim3(kScatterThreads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, kern, A) != cudaSuccess) {
-      cudaGetLastError();  // the passes one by one instead
-      return false;
-    }
-    COUNT_LAUNCH();
-    return true;
+    const dim3 grid((unsigned)((n + 512 * per - 1) / (512 * per)));
+    return launch_cooperative(c, kern, grid, kScatterThreads, (size_t)smem, s, A);
   };
   const int64_t rows = (n + 511) / 512;
   // sort phase, us, tiles of 1,024 / 2,048 / 4,096 keys: 4,099 keys 57 / 65 / 78,
@@ -1863,24 +1835,11 @@ constexpr int kUpWide = 30000;
 static void upward_pass(Ctx* c, const UpArgs& U, cudaStream_t s) {
   int64_t widest = 0;
   for (int L = 0; L <= kMaxLevel; ++L) widest = std::max<int64_t>(widest, c->lvl_host[L]);
-  if (widest <= kUpFusedWidest) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)std::min<int64_t>((widest + kUpThreads / 8 - 1) / (kUpThreads / 8),
-                                                   widest > 16384 ? 592 : 296));
-    cfg.blockDim = dim3(kUpThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_upward_all, c->max_level - 1, U, c->barrier(1, c->d_tree_status)) ==
-        cudaSuccess) {
-      COUNT_LAUNCH();
-      return;
-    }
-    cudaGetLastError();  // level by level instead
-  }
+  const dim3 grid((unsigned)std::min<int64_t>((widest + kUpThreads / 8 - 1) / (kUpThreads / 8),
+                                              widest > 16384 ? 592 : 296));
+  if (widest <= kUpFusedWidest && launch_cooperative(c, k_upward_all, grid, kUpThreads, 0, s, c->max_level - 1, U,
+                                                     c->barrier(1, c->d_tree_status)))
+    return;
   for (int L = c->max_level - 1; L >= 0; --L) {
     const int64_t cnt = c->lvl_host[L];
     if (cnt <= 0) continue;
@@ -1969,7 +1928,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
   // the host needs the node count M (grid sizes, allocations), the box, the level
   // counts and the status: the scan's last block writes them to mapped host memory
   exclusive_scan2<int32_t>(c->cstart.p, c->sstart.p, c->cend.p, c->send.p, n, c->scan_tmp.p, s,
-                           c->barrier(4, c->d_status),
+                           c, c->barrier(4, c->d_status),
                            SummaryArgs{c->d_box, c->d_small, c->d_status, c->lvlcnt, c->d_sum});
   if (!cuda_ok(c, cudaEventRecord(c->sum_ev, s), "grow summary")) return PEPCG_ERR_CUDA;
   cudaEventRecord(c->ev[9], s);
@@ -2040,7 +1999,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
   // count; the deepest twig level is one above the deepest leaf level
   {
     exclusive_scan2<int32_t>(bt, bt, ba, ba, (int64_t)nlb, c->scan_tmp.p, s,
-                             c->barrier(5, c->d_tree_status));
+                             c, c->barrier(5, c->d_tree_status));
     COUNT_LAUNCH();
     int32_t* cc = c->tcounts.p;
     int32_t* tcn = c->tcounts.p + ntw;
@@ -2048,7 +2007,7 @@ int grow_device(Ctx* c, int64_t n, const double* dx, const double* dy, const dou
                                             c->nc4.p, c->drec.p, c->lvlpos.p, c->child8.p,
                                             c->nchild.p, c->tinfo.p, cc, tcn, c->d_tree_status);
     exclusive_scan2<int32_t>(cc, cc, tcn, tcn, ntw, c->scan_tmp.p, s,
-                             c->barrier(6, c->d_tree_status));
+                             c, c->barrier(6, c->d_tree_status));
     UpArgs U{c->lvlcnt, c->twiglist.p, c->tinfo.p, cc, tcn, c->nleaves.p, c->drec.p,
              c->dmom.p, c->nc4.p, c->mom.p, reinterpret_cast<float4*>(c->mom32.p), c->d_tree_status};
     upward_pass(c, U, s);

@@ -59,7 +59,7 @@ struct DBuf {
 struct Walk;
 
 // what a context treats as refused by the driver (pepcg_debug_refuse, for tests)
-enum : uint32_t { kRefuseWalkStream = 1u << 0 };
+enum : uint32_t { kRefuseWalkStream = 1u << 0, kRefuseCooperative = 1u << 1, kRefuseCluster = 1u << 2 };
 
 // Per-node records are whole 32-byte sectors, so that the upward pass writes
 // no partial sector (a partial sector costs HBM a read-modify-write):
@@ -311,6 +311,29 @@ struct Ctx {
   unsigned barrier_tries = kBarrierTries;  // tests lower it (pepcg_debug_barrier_tries)
   GridBarrier barrier(int k, uint32_t* status) { return GridBarrier{barrier_word(k), status, barrier_tries}; }
 };
+
+// Cooperative launch; false: refused, the caller takes its other form.
+template <class... K, class... A>
+bool launch_cooperative(Ctx* c, void (*kern)(K...), dim3 grid, int threads, size_t smem, cudaStream_t s,
+                        const A&... args) {
+  if (c->refuse & kRefuseCooperative) return false;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, args...) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  COUNT_LAUNCH();
+  return true;
+}
 
 // The lanes of one pack of the packed per-tile walks: pack b holds the whole
 // tiles in targets [pstart[b], pstart[b + 1]), at most 32, and tflag gives

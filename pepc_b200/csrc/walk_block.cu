@@ -573,13 +573,12 @@ __global__ void __launch_bounds__(32 * W, W == 16 ? 1 : (W == 8 ? 2 : 4))
   warp_add3(A.counters, c_leaf, c_twig, c_mac);
 }
 
-// grid of `blocks` blocks in clusters of nparts
+// grid of `blocks` blocks in clusters of nparts; false: refused (the launchers below pass
+// it on, and the walk goes by one warp per bucket)
 template <class K, class A>
 bool launch_block(Ctx* c, K kern, int threads, size_t smem, int blocks, int nparts, cudaStream_t s,
                   const A& args, int* stack, int sweep) {
-  if (!cuda_ok(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-               "block walk"))
-    return false;
+  if ((c->refuse & kRefuseCluster) && nparts > 1) return false;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3((unsigned)threads);
@@ -591,8 +590,13 @@ bool launch_block(Ctx* c, K kern, int threads, size_t smem, int blocks, int npar
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = nparts > 1 ? 1 : 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaLaunchKernelEx(&cfg, kern, args, stack, nparts, sweep) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
   COUNT_LAUNCH();
-  return cuda_ok(c, cudaLaunchKernelEx(&cfg, kern, args, stack, nparts, sweep), "block walk");
+  return true;
 }
 
 }  // namespace

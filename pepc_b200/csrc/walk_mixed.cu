@@ -1077,7 +1077,7 @@ int launch_walk_mixed(Ctx* c, int64_t nt, const double* tx, const double* ty, co
   if (group64 && block_walk_shape(shape_nt, c->n, strict ? BlockWalk::kStrict : BlockWalk::kDefault, &sh)) {
     const size_t per = (size_t)148 * 5 * kWW * kStackCap;
     if (!ensure(c, c->wstack, 2 * per, "walk stacks")) return PEPCG_ERR_OOM;
-    return launch_walk_block64(c, A, sh, strict, c->wstack.p + slot * per, s) ? PEPCG_OK : PEPCG_ERR_CUDA;
+    if (launch_walk_block64(c, A, sh, strict, c->wstack.p + slot * per, s)) return PEPCG_OK;
   }
   COUNT_LAUNCH();
   if (per_target) {
@@ -1136,8 +1136,9 @@ int launch_adjoint_group64(Ctx* c, int64_t nt, const double* tx, const double* t
   const size_t per = (size_t)gblocks * kWW * kStackCap;
   if (!ensure(c, c->wstack, 2 * per, "walk stacks")) return PEPCG_ERR_OOM;
   BlockShape sh;
-  if (block_walk_shape(nt, c->n, BlockWalk::kAdjoint, &sh))
-    return launch_adj_block64(c, A, sh, with_e, c->wstack.p, s) ? PEPCG_OK : PEPCG_ERR_CUDA;
+  if (block_walk_shape(nt, c->n, BlockWalk::kAdjoint, &sh) &&
+      launch_adj_block64(c, A, sh, with_e, c->wstack.p, s))
+    return PEPCG_OK;
   COUNT_LAUNCH();
   if (with_e)
     k_adj_group64<true><<<gblocks, kMixThreads, 0, s>>>(A, c->wstack.p);

@@ -224,3 +224,55 @@ def test_refused_walk_stream_then_recovery(gpu, precision):
     assert all(np.array_equal(out[0][k], out[1][k]) for k in ("ex", "ey", "ez", "pot", "work"))
     tc.close()
     ref.close()
+
+
+def tree_bits(t):
+    return {k: (v.view(np.int64) if v.dtype == np.float64 else v) for k, v in t.tree().items()}
+
+
+# sizes: each tile width of the one-launch sort and both forms of the upward pass
+@pytest.mark.parametrize("n", [1000, 16411, 100003, 600001])
+def test_refused_cooperative_launches_give_the_same_tree(gpu, n):
+    x, y, z, q = cube(n, 92, charges="normal")
+    tc, ref = P.TreeCode(theta2=0.36, eps2=1e-4), P.TreeCode(theta2=0.36, eps2=1e-4)
+    P.lib().pepcg_debug_refuse(tc._h, 2)
+    launches, got = [], []
+    for t in (ref, tc):
+        a = P.lib().pepcg_kernel_launches()
+        g = t.pepc_grow_tree(x, y, z, q)
+        launches.append(P.lib().pepcg_kernel_launches() - a)
+        got.append((g.key, g.perm, tree_bits(t), t.sort_keys(g.key[::-1]),
+                    t.traverse_adjoint(x[:300], y[:300], z[:300], [np.zeros(300)] * 3, np.ones(300), n)))
+    assert launches[1] > launches[0]
+    a, b = got
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    assert all(np.array_equal(a[2][k], b[2][k]) for k in a[2])
+    assert all(np.array_equal(u, v) for u, v in zip(a[3], b[3]))
+    for k in a[4]:  # FP64 atomics, as above
+        assert np.abs(a[4][k] - b[4][k]).max() <= 1e-9 * np.abs(a[4][k]).max(), k
+    tc.close()
+    ref.close()
+
+
+# clusters of eight blocks of sixteen and of eight warps, of four blocks
+@pytest.mark.parametrize("n,nt", [(40000, 1000), (5000, 1000), (5000, 2000), (5000, 4000)])
+@pytest.mark.parametrize("precision", [P.PRECISION_MIXED, P.PRECISION_MIXED_STRICT])
+def test_refused_cluster_launches_walk_by_warps(gpu, precision, n, nt):
+    x, y, z, q = cube(n, 93, charges="normal")
+    t = np.random.default_rng(94).random((3, nt))
+    kw = dict(theta2=0.25, eps2=1e-4, precision=precision, walk=P.WALK_GROUP)
+    got = []
+    for refuse in (0, 4):
+        tc = P.TreeCode(**kw)
+        P.lib().pepcg_debug_refuse(tc._h, refuse)
+        tc.pepc_grow_tree(x, y, z, q)
+        got.append((tc.pepc_traverse_tree(*t),
+                    tc.traverse_adjoint(*t, [np.zeros(nt)] * 3, np.ones(nt), n)))
+        tc.close()
+    # the same lists (one opening test); the sums differ in order: FP32 within batches of
+    # 32, a few 2^-24 of terms that may cancel to a hundredth
+    (f, a), (g, b) = got
+    assert np.array_equal(f["work"], g["work"])
+    for u, v, keys in ((f, g, ("ex", "ey", "ez", "pot")), (a, b, ("q", "x", "y", "z"))):
+        for k in keys:
+            assert np.abs(u[k] - v[k]).max() <= 1e-5 * np.abs(u[k]).max(), k
