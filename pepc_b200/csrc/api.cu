@@ -699,7 +699,8 @@ int pepcg_traverse_tree(void* ctx, int64_t nt, const double* tx, const double* t
       return okd;
     };
     int rc = traverse_device(c, nt, b, b + nt, b + 2 * nt, nullptr, false, b + 3 * nt,
-                             b + 4 * nt, b + 5 * nt, b + 6 * nt, b + 7 * nt, nullptr, &plan);
+                             b + 4 * nt, b + 5 * nt, b + 6 * nt, b + 7 * nt, nullptr, &plan, 0,
+                             tkeys != nullptr);
     const bool drained = drain_copies(c, true);
     if (rc && rc != PEPCG_WARN_NOT_NEUTRAL) return rc;
     return drained ? rc : PEPCG_ERR_CUDA;

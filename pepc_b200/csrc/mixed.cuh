@@ -703,7 +703,7 @@ struct BlockShape {
 // A bucket's sums depend on the shape only (FP32 batches), so calls that must
 // give the same fields pass the same nt here.
 enum class BlockWalk { kDefault, kStrict, kAdjoint };
-bool block_walk_shape(int64_t nt, int64_t npart, BlockWalk kind, BlockShape* sh);
+bool block_walk_shape(int64_t nt, int64_t npart, BlockWalk kind, bool keyed, BlockShape* sh);
 bool launch_walk_block64(Ctx* c, const MixArgs& A, const BlockShape& sh, bool strict, int* stack,
                          cudaStream_t s);
 bool launch_adj_block64(Ctx* c, const AdjMixArgs& A, const BlockShape& sh, bool with_e, int* stack,

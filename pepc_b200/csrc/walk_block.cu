@@ -611,9 +611,20 @@ bool launch_block(Ctx* c, K kern, int threads, size_t smem, int blocks, int npar
 // 0.33, 938: 0.52 against 0.58).  The adjoint: 4,688 buckets 6.2 against 6.7 ms.
 // Few buckets on a large tree are scattered targets with long lists: sixteen warps
 // and eight blocks (8 buckets, 262,144 sources: 0.135 against 0.18 ms).
-bool block_walk_shape(int64_t nt, int64_t npart, BlockWalk kind, BlockShape* sh) {
+// Walked targets without keys (keyed false) may lie in any order, and buckets of
+// scattered targets are alike: the walk by warps then loses nothing to a longest bucket,
+// only to its last wave.  Random and evenly spread targets, targets on a line, of or among
+// 100,000 and 1M particles, theta 0.4 and 0.6, time by warps / by blocks:
+//   default form  4,063 buckets 0.90 .. 1.05, 4,400: 0.95 .. 1.07, 5,469: 0.94 .. 1.12, 8,594:
+//                 0.92 .. 1.02; up to 4,096 none of the cells is slower than the walk by
+//                 warps was before both were tuned, from 4,400 some are (0.94 .. 0.97);
+//   strict form   2,200 buckets 1.01 .. 1.31, 2,300: 0.92 .. 1.14, 2,368, which fill one wave of
+//                 its resident warps: 0.92 .. 1.13, 2,375: 0.99 .. 1.29, 2,960: 1.00 .. 1.19.
+bool block_walk_shape(int64_t nt, int64_t npart, BlockWalk kind, bool keyed, BlockShape* sh) {
   const int64_t nb = (nt + 63) / 64;
-  if (nb > (kind == BlockWalk::kStrict ? 5000 : kind == BlockWalk::kAdjoint ? 6000 : 9000)) return false;
+  if (nb > (kind == BlockWalk::kStrict ? 5000 : kind == BlockWalk::kAdjoint ? 6000 : keyed ? 9000 : 4096))
+    return false;
+  if (kind == BlockWalk::kStrict && !keyed && nb > 2200 && nb <= 148 * 4 * kWW) return false;
   if (nb <= 18 && npart >= 32768) *sh = {16, 8};
   else if (nb <= 37) *sh = {8, 8};
   else if (nb <= 74) *sh = {8, 4};

@@ -1038,7 +1038,7 @@ int launch_walk_mixed(Ctx* c, int64_t nt, const double* tx, const double* ty, co
                       double* ex, double* ey, double* ez, double* pot, double* work,
                       const int2* tiles, int64_t ntiles, bool per_target,
                       const int32_t* tflag, const int32_t* pstart, const int32_t* npacks,
-                      cudaStream_t s, int slot, int64_t shape_nt) {
+                      cudaStream_t s, int slot, int64_t shape_nt, bool keyed) {
   MixArgs A;
   A.nt = nt;
   A.tx = tx; A.ty = ty; A.tz = tz;
@@ -1074,7 +1074,7 @@ int launch_walk_mixed(Ctx* c, int64_t nt, const double* tx, const double* ty, co
   BlockShape sh;
   const bool group64 = !per_target && !tflag && tiles == nullptr && c->group_size() == 64;
   const bool strict = c->prm.precision == PEPCG_PRECISION_MIXED_STRICT;
-  if (group64 && block_walk_shape(shape_nt, c->n, strict ? BlockWalk::kStrict : BlockWalk::kDefault, &sh)) {
+  if (group64 && block_walk_shape(shape_nt, c->n, strict ? BlockWalk::kStrict : BlockWalk::kDefault, keyed, &sh)) {
     const size_t per = (size_t)148 * 5 * kWW * kStackCap;
     if (!ensure(c, c->wstack, 2 * per, "walk stacks")) return PEPCG_ERR_OOM;
     if (launch_walk_block64(c, A, sh, strict, c->wstack.p + slot * per, s)) return PEPCG_OK;
@@ -1136,7 +1136,7 @@ int launch_adjoint_group64(Ctx* c, int64_t nt, const double* tx, const double* t
   const size_t per = (size_t)gblocks * kWW * kStackCap;
   if (!ensure(c, c->wstack, 2 * per, "walk stacks")) return PEPCG_ERR_OOM;
   BlockShape sh;
-  if (block_walk_shape(nt, c->n, BlockWalk::kAdjoint, &sh) &&
+  if (block_walk_shape(nt, c->n, BlockWalk::kAdjoint, false, &sh) &&
       launch_adj_block64(c, A, sh, with_e, c->wstack.p, s))
     return PEPCG_OK;
   COUNT_LAUNCH();

@@ -899,7 +899,7 @@ int launch_walk_mixed(Ctx* c, int64_t nt, const double* tx, const double* ty, co
                       double* ex, double* ey, double* ez, double* pot, double* work,
                       const int2* tiles, int64_t ntiles, bool per_target, const int32_t* tflag,
                       const int32_t* pstart, const int32_t* npacks, cudaStream_t s, int slot,
-                      int64_t shape_nt);
+                      int64_t shape_nt, bool keyed);
 
 const double* grown_charges_if_same(Ctx* c, int64_t nt, const int64_t* d_tkeys) {
   if (!d_tkeys || nt != c->n) return nullptr;
@@ -987,6 +987,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
              "with the grown keys)";
     return PEPCG_ERR_UNSUPPORTED;
   }
+  keyed = keyed || self || tkeys;
   cudaStream_t s = c->stream;
   const int walk = c->prm.walk;
   // bucket queues, counters, barrier words and the status word
@@ -1106,7 +1107,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
   A.has_cut = has_spatial_cutoff(c->prm) ? 1 : 0;
   for (int k = 0; k < 3; ++k) A.cut[k] = c->prm.spatial_interaction_cutoff[k];
   const int blocks = 148 * 8;
-  const bool lists = use_list_walk(c, nt, self || tkeys || keyed, plan != nullptr, packed);
+  const bool lists = use_list_walk(c, nt, keyed, plan != nullptr, packed);
   if (lists) {
     A.lper = list_bucket(nt);
     const int64_t nbk = packed ? (nt + kPackChunk - 1) / kPackChunk * kPackSlots
@@ -1181,7 +1182,7 @@ int traverse_device(Ctx* c, int64_t nt, const double* tx, const double* ty, cons
         int rc = launch_walk_mixed(c, t1 - t0, A.tx, A.ty, A.tz, A.ex, A.ey, A.ez, A.pot, A.work,
                                    walk == PEPCG_WALK_PER_TILE ? A.tiles : nullptr, ntiles,
                                    walk == PEPCG_WALK_PER_TARGET, packed ? c->tflag.p : nullptr,
-                                   pstart, npacks, sk, slot, shape_nt > 0 ? shape_nt : nt);
+                                   pstart, npacks, sk, slot, shape_nt > 0 ? shape_nt : nt, keyed);
         if (rc) return rc;
       }
       if (!cuda_ok(c, cudaGetLastError(), "walk launch")) return PEPCG_ERR_CUDA;

@@ -77,6 +77,30 @@ def test_block_walk_matches_fp64_lists(gpu, n, periodic):
     plain.close()
 
 
+@pytest.mark.parametrize("precision,lines", [(P.PRECISION_MIXED, (4096, 9000)),
+                                             (P.PRECISION_MIXED_STRICT, (2200, 2368, 5000))])
+def test_targets_with_and_without_keys(gpu, precision, lines):
+    # without keys other bucket counts go by blocks: the same lists, and sums that differ in
+    # order (FP32 in batches of 32, then FP64: a few 2^-24 of terms that cancel to a tenth)
+    p, _ = sources(2500, 15)
+    tc = context(p, precision=precision, theta2=0.25, eps2=1e-4)
+    q = [torch.empty(2500, dtype=torch.float64, device="cuda") for _ in range(4)]
+    k = torch.empty((2, 2500), dtype=torch.int64, device="cuda")
+    tc.particles_device(*k, *q)
+    for nb in lines:
+        for nt in (64 * nb - 63, 64 * nb + 1):
+            i = torch.arange(nt, device="cuda") * 2500 // nt  # in key order
+            t, keys = [a[i].contiguous() for a in q[:3]], k[0][i].contiguous()
+            a = fields(tc, t)
+            b = torch.zeros_like(a)
+            tc.traverse_tree_device(*t, *b, keys=keys)
+            assert torch.equal(a[4], b[4]), nt
+            scale = a[:3].norm(dim=0).median()
+            off = (a[:3] - b[:3]).norm(dim=0) / torch.maximum(a[:3].norm(dim=0), scale)
+            assert float(off.max()) < 5e-6, (nt, float(off.max()))
+    tc.close()
+
+
 @pytest.mark.parametrize("with_e", [False, True])
 @pytest.mark.parametrize("n", [2500, 33000])
 def test_block_adjoint_matches_fp64(gpu, n, with_e):
