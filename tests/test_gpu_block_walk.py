@@ -55,8 +55,8 @@ def test_block_walk_matches_fp64_lists(gpu, n, periodic):
     for prec in (P.PRECISION_MIXED, P.PRECISION_MIXED_STRICT):
         tc = context(p, precision=prec, **kw)
         for nt in EDGES:
-            if nt > 10000 and (periodic or n > 10000):
-                continue
+            if nt > 40000 and (periodic or n > 10000):
+                continue  # 38,401 targets, the first count of four-warp blocks, are in
             t = targets(nt, g)
             a, b = fields(plain, t), fields(tc, t)
             if prec == P.PRECISION_MIXED_STRICT:
@@ -109,7 +109,7 @@ def test_block_adjoint_matches_fp64(gpu, n, with_e):
     plain = context(p, precision=P.PRECISION_PLAIN, **kw)
     tc = context(p, precision=P.PRECISION_MIXED, **kw)
     for nt in EDGES + [6000 * 64 + 1]:
-        if nt > 10000 and n > 10000:
+        if nt > 40000 and n > 10000:
             continue
         t = targets(nt, g)
         gr = torch.randn((4, nt), generator=g, dtype=torch.float64, device="cuda")
@@ -155,4 +155,28 @@ def test_bucket_results_accumulate(gpu):
     tc.traverse_tree_device(*t, *twice)
     assert torch.equal(twice[4], 2 * once[4])
     assert float((twice - 2 * once).abs().max()) <= 1e-12 * float(once.abs().max())
+    tc.close()
+
+
+def test_more_nodes_than_a_packed_stack_entry_holds(gpu):
+    # above 2^25 nodes the image boxes are swept one after the other: the fields of 27 boxes
+    # against 27 walks of the open tree by shifted targets (the same lists but where the
+    # shift's rounding decides a node otherwise)
+    n = 24_000_000
+    p, g = sources(n, 16)
+    kw = dict(precision=P.PRECISION_MIXED, theta2=0.25, eps2=1e-6)
+    targets_of = [targets(nt, g) for nt in (500, 9000)]  # clusters, and one block per bucket
+    tc = context(p, periodicity=(1, 1, 1), include_far_field_if_periodic=0, **kw)
+    assert P.lib().pepcg_num_nodes(tc._h) > 2 ** 25
+    boxes = [fields(tc, t) for t in targets_of]
+    tc.close()
+    tc = context(p, **kw)
+    for t, a in zip(targets_of, boxes):
+        b = torch.zeros_like(a)
+        for i in range(27):
+            tc.traverse_tree_device(*[c + (i // 3 ** k % 3 - 1) for k, c in enumerate(t)], *b)
+        assert float(((a[4] - b[4]).abs() / b[4]).max()) < 1e-3
+        off = (a[:3] - b[:3]).norm(dim=0) / b[:3].norm(dim=0).median()
+        assert float(off.median()) < 2e-6, float(off.median())
+        assert float(off.max()) < 5e-4, float(off.max())
     tc.close()
