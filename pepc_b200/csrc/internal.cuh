@@ -260,7 +260,7 @@ struct Ctx {
   int nboxes = 1;
   double vbox[3 * 125];      // lattice vectors of the near-field boxes, central last
   double* d_vbox = nullptr;   // the same on the device
-  double* d_part = nullptr;   // bbox partials (6 * 296)
+  double* d_part = nullptr;   // bbox partials (6 * 512)
   double2* d_mlattice = nullptr;  // 861 complex
   // expansions of order 20 (231 orders): the harmonics' recurrence and leading
   // factors, the force coefficients from mu, block partials of the particle sums,

@@ -1,11 +1,12 @@
 // walk_block.cu -- the 64-target group walk and its adjoint with one thread
-// block (or a cluster of blocks) per target bucket, for walks whose buckets are
-// too few to give every warp of the chip one of its own.
+// block (or a cluster of blocks) per target bucket, for walks of few buckets
+// (block_walk_shape has the lines).
 //
 // k_walk_group64 and k_adj_group64 (walk_mixed.cu) give each bucket to one warp,
 // whose traversal is a serial chain of dependent loads and batches: with fewer
 // buckets than resident warps (2,960) most of the chip idles and the call takes
-// the longest bucket's chain.  Here the W warps of a block share one bucket:
+// the longest bucket's chain, and with up to three times as many buckets in key order
+// the last of them still do.  Here the W warps of a block share one bucket:
 //  - one traversal stack per block (global memory): a round pops up to 32 W
 //    nodes, one per thread, decided exactly as there (the same FP32
 //    group-centred opening test), so the lists are the same;
@@ -38,7 +39,6 @@ constexpr int kBoxShift = 25;     // stack entry: node | box << 25 (trees below 
 // what the traversal reads, of either kernel's arguments
 struct BlockTree {
   const LevelRecord* drec;
-  const float4* mom32;
   const double* macb;
   float theta2;
   double theta2d;
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(32 * W, walk_block_resident<W, kStrict>())
   int* stack = gstack + (int64_t)blockIdx.x * W * kStackCap;
   const int part = nparts > 1 ? (int)(blockIdx.x % nparts) : 0;
   const int64_t nbuckets = *A.tree_status & ST_TIMEOUT ? 0 : (A.nt + 63) / 64;
-  const BlockTree B{A.drec, A.mom32, A.macb, A.theta2, A.theta2d};
+  const BlockTree B{A.drec, A.macb, A.theta2, A.theta2d};
   unsigned long long c_leaf = 0, c_twig = 0, c_mac = 0;
   for (bool first = true;; first = false) {
     // a bucket from the queue, or (clusters: one bucket each) the cluster's
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(32 * W, W == 16 ? 1 : (W == 8 ? 2 : 4))
   int* stack = gstack + (int64_t)blockIdx.x * W * kStackCap;
   const int part = nparts > 1 ? (int)(blockIdx.x % nparts) : 0;
   const int64_t nbuckets = (A.nt + 63) / 64;
-  const BlockTree B{A.drec, A.mom32, A.macb, A.theta2, 0.0};
+  const BlockTree B{A.drec, A.macb, A.theta2, 0.0};
   const float2 E2 = f2(A.eps2);
   unsigned long long c_leaf = 0, c_twig = 0, c_mac = 0;
   for (bool first = true;; first = false) {

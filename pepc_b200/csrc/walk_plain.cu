@@ -928,8 +928,9 @@ int prepare_mac(Ctx* c, const double** macb) {
   return PEPCG_OK;
 }
 
-// Whether the plain walk of nt targets goes by k_walk_list64: while its buckets are
-// fewer than the warps that the walks by warp keep resident (2,368), and where a list
+// Whether the plain walk of nt targets goes by k_walk_list64: while its buckets of 32
+// are fewer than the warps that the walks by warp keep resident (2,960 per target, 96
+// registers and five blocks of four warps per SM; 3,552 per tile), and where a list
 // is likely to fit (theta >= 0.35, or a tree smaller than a list).  Walk ms, by warp ->
 // by lists, per target: 1,000 particles 0.237 -> 0.082, 4,099: 0.46 -> 0.117, 16,411
 // (Plummer, theta 0.4) 3.36 -> 1.22, 40,009: 0.86 -> 0.56; per tile 4,099: 0.46 -> 0.133, 40,009:
