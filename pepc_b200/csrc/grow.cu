@@ -916,11 +916,12 @@ __global__ void k_gather(int64_t n, const int32_t* __restrict__ sval,
                          const double* __restrict__ box, int curve,
                          const uint32_t* __restrict__ status) {
   const unsigned long long nd = *dupcount;
-  if (*status & ST_TIMEOUT) return;  // no sorted indices
+  const uint32_t st = *status;
   const bool fixed = nd > 0 && nd <= (unsigned long long)dupcap;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int32_t j = sval[i];
+    if (st & ST_TIMEOUT) return;  // no sorted indices (tested here: the loads go out together)
     double4 p = ld256(packed + j);
     if (fixed && key[i] != korig[i]) {
       int64_t ic[3];

@@ -99,27 +99,31 @@ __device__ __forceinline__ void st256f(void* p, float4 a, float4 b) {
 // bounded (seconds): a block whose tries run out closes the word, unless the
 // barrier completes first, and no block passes a closed one: the status word gets
 // ST_TIMEOUT, every thread of every block sees false and returns.  So what a kernel
-// writes after its last barrier is written by all its blocks or by none.  No tries at
-// all (tests): the first block to arrive closes the word.
+// writes after its last barrier is written by all its blocks or by none.
 constexpr unsigned kBarrierTries = 1u << 22;
 constexpr unsigned kBarrierClosed = 1u << 31;
 struct GridBarrier {
   unsigned* word;
   uint32_t* status;
   unsigned tries;
+  unsigned never;  // tests: added to the target, which is then never reached
 };
 __device__ __forceinline__ bool grid_barrier(const GridBarrier& B, unsigned target) {
   __syncthreads();
   int late = 0;
   if (threadIdx.x == 0) {
     __threadfence();
-    unsigned seen = B.tries ? atomicAdd(B.word, 1u) + 1u
-                            : atomicOr(B.word, kBarrierClosed) | kBarrierClosed;
-    for (unsigned t = 0; seen < target && t < B.tries; ++t)
+    atomicAdd(B.word, 1u);
+    target += B.never;
+    unsigned seen = 0;
+    for (unsigned t = 0;;) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(B.word) : "memory");
-    while (seen < target) {  // a failed exchange is another block's arrival
-      const unsigned old = atomicCAS(B.word, seen, seen | kBarrierClosed);
-      seen = old == seen ? seen | kBarrierClosed : old;
+      if (seen >= target) break;
+      // out of tries: a failed exchange is another block's arrival
+      if (++t >= B.tries && atomicCAS(B.word, seen, seen | kBarrierClosed) == seen) {
+        seen = kBarrierClosed;
+        break;
+      }
     }
     if (seen & kBarrierClosed) {
       late = 1;
@@ -309,7 +313,9 @@ struct Ctx {
   unsigned int* barrier_word(int k) { return reinterpret_cast<unsigned int*>(d_small + 16) + k; }
   uint32_t refuse = 0;                     // kRefuse bits (pepcg_debug_refuse)
   unsigned barrier_tries = kBarrierTries;  // tests lower it (pepcg_debug_barrier_tries)
-  GridBarrier barrier(int k, uint32_t* status) { return GridBarrier{barrier_word(k), status, barrier_tries}; }
+  GridBarrier barrier(int k, uint32_t* status) {
+    return GridBarrier{barrier_word(k), status, barrier_tries, barrier_tries ? 0u : 1u << 30};
+  }
 };
 
 // Cooperative launch; false: refused, the caller takes its other form.
