@@ -623,7 +623,7 @@ void sort_pass(int64_t n, const uint64_t* kin, const int32_t* vin, uint64_t* kou
 // All LSD passes in one cooperative launch, for arrays of few tiles.
 //
 // Up to 148 tiles the 28 launches of the passes above are short of work: at
-// 16,411 keys the sort phase took 172 us with them and takes 68 us with this, most of
+// 16,411 keys the sort phase took 172 us with them and takes 65 us with this, most of
 // the difference the start and end of kernels that run for 1-2 us.  Here every tile has a resident block that keeps it through all
 // passes, with two grid barriers per pass: one once the tiles' digit counts are
 // written, after which each block sums the count columns itself (thread d digit d,
@@ -1760,7 +1760,9 @@ static bool coop_sort(Ctx* c, int64_t n, int dupcap, cudaStream_t s) {
   const int64_t rows = (n + 511) / 512;
   // sort phase, us, tiles of 1,024 / 2,048 / 4,096 keys: 4,099 keys 57 / 65 / 78,
   // 16,411: 68 / 69 / 88, 60,013: 90 / 90 / 102, 100,003: 107 / 94 / 100, 200,003: - / 123
-  // / 116, 600,000: - / - / 166 (the passes one by one: 164, 172, 172, 172, 177, 184)
+  // / 116, 600,000: - / - / 166 (the passes one by one: 164, 172, 172, 172, 177, 184);
+  // the chosen ones since the barrier's give-up test moved into its polling loop: 57, 65, 85,
+  // 85, 105, 142
   const int per = rows <= 64 ? 2 : rows <= 256 ? 4 : 8;
   if ((rows + per - 1) / per > kCoopTiles) return false;
   if (per == 2) return go(k_sort_coop<kGrow, 2>, 2, coop_smem<2>());

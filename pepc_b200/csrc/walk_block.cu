@@ -617,8 +617,8 @@ bool launch_block(Ctx* c, K kern, int threads, size_t smem, int blocks, int npar
 // 100,000 and 1M particles, theta 0.4 and 0.6, time by warps / by blocks:
 //   default form  4,063 buckets 0.90 .. 1.05, 4,400: 0.95 .. 1.07, 5,469: 0.94 .. 1.12, 8,594:
 //                 0.92 .. 1.02; up to 4,096 none of the cells is slower than the walk by
-//                 warps was before both were tuned, from 4,400 some are (0.94 .. 0.97);
-//   strict form   2,200 buckets 1.01 .. 1.31, 2,300: 0.92 .. 1.14, 2,368, which fill one wave of
+//                 warps was before both were tuned, from 4,400 some are (0.93 .. 0.97);
+//   strict form   2,200 buckets 1.01 .. 1.20, 2,300: 0.92 .. 1.14, 2,368, which fill one wave of
 //                 its resident warps: 0.92 .. 1.13, 2,375: 0.99 .. 1.29, 2,960: 1.00 .. 1.19.
 bool block_walk_shape(int64_t nt, int64_t npart, BlockWalk kind, bool keyed, BlockShape* sh) {
   const int64_t nb = (nt + 63) / 64;
